@@ -1,4 +1,5 @@
-// Register-resident DFT codelets for radix 2, 3, 4, 5, 7, 8, 9, 16 and 25, and the complex helpers the pass kernels use.
+// Register-resident DFT codelets for radix 2, 3, 4, 5, 7, 8, 9, 16, 25, 32 and the products of coprime ones (6 .. 24), and
+// the complex helpers the pass kernels use.
 //
 // These replace the reference's machine-generated straight-line SIMD codelets (engine/numerics/hesap-fft/kernels/
 // fft_*_codelets_*.cpp, emitted by scripts/gen_fft_batched.py and scripts/gen_fft_codelets.py) and add the odd radices
@@ -83,6 +84,11 @@ template <int J, class C> __device__ __forceinline__ C w16mul(C a)
 }
 
 template <int R> struct Dft;
+
+template <> struct Dft<1>
+{
+    template <class C> __device__ __forceinline__ static void run(C*) {}
+};
 
 template <> struct Dft<2>
 {
@@ -407,6 +413,75 @@ template <> struct Dft<9>
                 v[k1 + 3 * k2] = b[k2];
         }
     }
+};
+
+// R = A B with A and B coprime: the prime-factor mapping (Good, Thomas). Input n = (B a + A b) mod R and output
+// k = (B B' ka + A A' kb) mod R with B B' = 1 mod A and A A' = 1 mod B give an A x B transform with no twiddles between
+// the two: every index is a compile-time register number.
+constexpr int inverse_mod(int a, int m)
+{
+    for (int i = 1; i < m; ++i)
+        if ((a * i) % m == 1)
+            return i;
+    return 1;
+}
+
+template <int A, int B> struct CoprimeDft
+{
+    template <class C> __device__ __forceinline__ static void run(C* v)
+    {
+        constexpr int R = A * B;
+        constexpr int ca = B * inverse_mod(B % A, A), cb = A * inverse_mod(A % B, B);
+        C t[B][A];
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+        {
+#pragma unroll
+            for (int a = 0; a < A; ++a)
+                t[b][a] = v[(B * a + A * b) % R];
+            Dft<A>::run(t[b]);
+        }
+#pragma unroll
+        for (int a = 0; a < A; ++a)
+        {
+            C u[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b)
+                u[b] = t[b][a];
+            Dft<B>::run(u);
+#pragma unroll
+            for (int b = 0; b < B; ++b)
+                v[(ca * a + cb * b) % R] = u[b];
+        }
+    }
+};
+
+template <> struct Dft<6> : CoprimeDft<2, 3>
+{
+};
+template <> struct Dft<10> : CoprimeDft<2, 5>
+{
+};
+template <> struct Dft<12> : CoprimeDft<4, 3>
+{
+};
+template <> struct Dft<14> : CoprimeDft<2, 7>
+{
+};
+template <> struct Dft<15> : CoprimeDft<3, 5>
+{
+};
+template <> struct Dft<18> : CoprimeDft<2, 9>
+{
+};
+template <> struct Dft<20> : CoprimeDft<4, 5>
+{
+};
+template <> struct Dft<21> : CoprimeDft<3, 7>
+{
+};
+template <> struct Dft<24> : CoprimeDft<8, 3>
+{
 };
 
 } // namespace crdfft

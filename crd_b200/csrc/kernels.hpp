@@ -17,6 +17,13 @@ namespace crdfft
 // One launch of the line-FFT kernel (line_fft.cu).
 cudaError_t launch_line_pass(const PassDesc& d, const PassShape& sh, const void* in, void* out, cudaStream_t stream);
 
+// The same pass for a length without a compile-time schedule (smooth_line.cu): the tile's lines, threads and shared
+// memory; the pass's radices are smooth_radices' and its twiddles theirs.
+bool smooth_line_supported(const PassDesc& d);
+int smooth_line_lpc(const PassDesc& d, PassMap map);
+int smooth_line_smem(const PassDesc& d, int lpc);
+cudaError_t launch_smooth_line(const PassDesc& d, int lpc, const void* in, void* out, cudaStream_t stream);
+
 // Fused FFT convolution of the lines of a pass (conv.cu): out = conj(FFT(conj(FFT(in) * H))) * scale, with H's
 // element e of line l at line_offset(smap, l) + e * smap.estride, the pass's conj_out set and its scale.
 bool conv_supported(const PassDesc& d);

@@ -1,5 +1,5 @@
 // Launchers of the line-FFT pass kernels (line_fft.cuh): the pipelined persistent kernel where the planner chose it,
-// else the compile-time schedule when one exists for the pass, else the run-time schedule.
+// else the compile-time schedule when one exists for the pass, else the run-time schedule (smooth_line.cu).
 
 #include "kernels.hpp"
 #include "line_fft.cuh"
@@ -104,7 +104,7 @@ bool pass_has_kernel(const PassDesc& d, const PassShape& sh)
         return row_tstore_supported(d, sh);
     if (sh.pipelined)
         return lfft::select_pipe(d, sh) != nullptr;
-    return lfft::select_static(d, sh) != nullptr || lfft::select_dynamic(d, sh) != nullptr;
+    return lfft::select_static(d, sh) != nullptr;
 }
 
 namespace
@@ -190,16 +190,9 @@ cudaError_t launch_line_pass(const PassDesc& d, const PassShape& sh, const void*
         cs.smem_bytes = sh.lines_per_cta * lfft::cta_line_pitch(d.n, sh.lines_per_cta) * 8;
     }
     lfft::KernelFn fn = lfft::select_static(d, cs);
-    if (fn == nullptr)
-    {
-        // the run-time schedule kernel always stages its lines through shared memory, in two buffers (even for a
-        // one-stage pass that a compile-time kernel runs register to register)
-        fn = lfft::select_dynamic(d, cs);
-        cs.smem_bytes = 2 * sh.lines_per_cta * lfft::line_pitch(d.n) * 8; // two line buffers: out-of-place stages
-        if (cs.smem_bytes > 227 * 1024)
-            return cudaErrorInvalidConfiguration;
-    }
-    if (fn == nullptr || threads > lfft::max_threads(sh.points_per_thread, d.n))
+    if (fn == nullptr) // no compile-time schedule
+        return launch_smooth_line(d, sh.lines_per_cta, in, out, stream);
+    if (threads > lfft::max_threads(sh.points_per_thread, d.n))
         return cudaErrorInvalidConfiguration;
     if (groups > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;

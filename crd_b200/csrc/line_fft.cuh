@@ -255,66 +255,6 @@ __device__ __forceinline__ void run_static(const PassDesc& d, const Ctx& c, cons
         run_static<P, DL, DS, PIPE, K, L * R, OFF + (L > 1 ? (R - 1) * L : 0), Rest...>(d, c, lay, n);
 }
 
-template <int R, int P, bool DL, bool DS, class K, class Lay>
-__device__ __forceinline__ void stage_dyn(const PassDesc& d, const Ctx& c, const Lay& lay, int n, int L, int off,
-                                          bool first, bool last)
-{
-    if constexpr (DL)
-    {
-        if (first)
-        {
-            if constexpr (DS)
-            {
-                if (last)
-                {
-                    stage<R, P, true, true, false, K>(d, c, lay, n, L, off);
-                    return;
-                }
-            }
-            stage<R, P, true, false, false, K>(d, c, lay, n, L, off);
-            return;
-        }
-    }
-    if constexpr (DS)
-    {
-        if (last)
-        {
-            stage<R, P, false, true, false, K>(d, c, lay, n, L, off);
-            return;
-        }
-    }
-    stage<R, P, false, false, false, K>(d, c, lay, n, L, off);
-}
-
-template <int P, bool DL, bool DS, class K, class Lay>
-__device__ __forceinline__ void run_dynamic(const PassDesc& d, const Ctx& c, const Lay& lay, int n)
-{
-    int L = 1;
-    int off = 0;
-    for (int s = 0; s < d.nstages; ++s)
-    {
-        const int R = d.radix[s];
-        const bool first = s == 0;
-        const bool last = s == d.nstages - 1;
-        switch (R)
-        {
-            case 2: stage_dyn<2, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-            case 3: stage_dyn<3, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-            case 4: stage_dyn<4, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-            case 5: stage_dyn<5, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-            case 7: stage_dyn<7, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-            case 9: stage_dyn<9, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-            case 25: stage_dyn<25, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-            case 8: stage_dyn<8, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-            case 32: stage_dyn<32, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-            default: stage_dyn<16, P, DL, DS, K>(d, c, lay, n, L, off, first, last); break;
-        }
-        if (L > 1)
-            off += (R - 1) * L;
-        L *= R;
-    }
-}
-
 template <class S> struct SchedRun
 {
     template <int P, bool DL, bool DS, bool PIPE, class K, class Lay>
@@ -328,16 +268,6 @@ template <class S> struct SchedRun
         run_static<P, DL, DS, PIPE, K, 1, 0, Rs...>(d, c, lay, n);
     }
 };
-template <> struct SchedRun<DynSched>
-{
-    template <int P, bool DL, bool DS, bool PIPE, class K, class Lay>
-    __device__ __forceinline__ static void go(const PassDesc& d, const Ctx& c, const Lay& lay, int n)
-    {
-        static_assert(!PIPE, "the pipelined kernel runs compile-time schedules only");
-        run_dynamic<P, DL, DS, K>(d, c, lay, n);
-    }
-};
-
 template <class S> __device__ __forceinline__ int sched_n(const PassDesc& d)
 {
     if constexpr (std::is_same_v<S, DynSched>)
@@ -942,11 +872,10 @@ inline bool same_radices(const PassDesc& d, std::initializer_list<int> rs)
         return nullptr;                                                                                                \
     }
 
-// Instances live in line_fft_static.cu (compile-time schedules, classic and pipelined) and line_fft_dyn.cu
-// (schedule read from the descriptor); each returns nullptr when it has no kernel for the pass.
+// Each returns nullptr when it has no kernel for the pass; the lengths without a compile-time schedule run
+// smooth_line.cu.
 KernelFn select_static(const PassDesc& d, const PassShape& sh);
 PipeFn select_pipe(const PassDesc& d, const PassShape& sh);
-KernelFn select_dynamic(const PassDesc& d, const PassShape& sh);
 
 } // namespace lfft
 } // namespace crdfft

@@ -18,6 +18,7 @@
 #include "../../include/crdfft.h"
 #include "kernels.hpp"
 #include "pass_desc.hpp"
+#include "smooth_plan.hpp"
 #include "tuner.hpp"
 #include "learned.hpp"
 #include "uneven.hpp"
@@ -293,7 +294,7 @@ struct Plan
     int device = 0;
     std::vector<Step> steps[2];
     std::vector<void*> tables;
-    std::map<long long, void*> tw_by_n;
+    std::map<std::vector<int>, void*> tw_by_radices;
     long long table_bytes = 0;
     size_t ws_bytes = 0;
     void* ws = nullptr;
@@ -457,24 +458,21 @@ void root(long long k, long long n, double* re, double* im)
     *im = static_cast<double>(-sr);
 }
 
-// The stage-ordered twiddle table of a line length n with the planner's radix schedule: for each stage after the
+// The stage-ordered twiddle table of a line length n under a radix schedule: for each stage after the
 // first (radix R, after radices multiplying to L), W_{LR}^{r k} = W_n^{r k n/(L R)} at (r-1) L + k. Each entry is
-// computed in FP64 and narrowed once (fft.hpp:251-260).
-crdfft_status twiddle_table(Plan& p, long long n, const void** out, bool r32 = false, bool group25 = true)
+// computed in FP64 and narrowed once (fft.hpp:251-260). One table per schedule and plan.
+crdfft_status twiddle_table(Plan& p, const std::vector<int>& rad, const void** out)
 {
-    // one table per (length, schedule family)
-    const long long key = n | (r32 ? (1LL << 48) : 0) | (group25 ? 0 : (1LL << 49));
-    auto it = p.tw_by_n.find(key);
-    if (it != p.tw_by_n.end())
+    auto it = p.tw_by_radices.find(rad);
+    if (it != p.tw_by_radices.end())
     {
         *out = it->second;
         return CRDFFT_OK;
     }
-    std::vector<int> rad;
-    if (!radices_for(n, rad, r32, group25))
-        return CRDFFT_UNSUPPORTED_SIZE;
     std::vector<float> h;
-    long long L = 1;
+    long long n = 1, L = 1;
+    for (int R : rad)
+        n *= R;
     for (int R : rad)
     {
         if (L > 1)
@@ -494,7 +492,7 @@ crdfft_status twiddle_table(Plan& p, long long n, const void** out, bool r32 = f
     const crdfft_status st = upload_table(p, h, &d);
     if (st != CRDFFT_OK)
         return st;
-    p.tw_by_n[key] = d;
+    p.tw_by_radices[rad] = d;
     *out = d;
     return CRDFFT_OK;
 }
@@ -521,6 +519,28 @@ PassShape shape_with(long long n, int nstages, PassMap map, bool dl, bool ds, in
         --lpc;
     sh.lines_per_cta = lpc;
     sh.smem_bytes = needs_smem ? tile_bytes(lpc) : 0;
+    return sh;
+}
+
+// The shape of a pass without a compile-time schedule (smooth_line.cu) at `lpc` lines a CTA (0: its default); the
+// threads follow from the lines and the radices.
+bool smooth_pass(const PassDesc& d)
+{
+    return !pass_has_static(d, 16) && !pass_has_static(d, 32) && smooth_line_supported(d);
+}
+
+PassShape smooth_shape(const PassDesc& d, PassMap map, bool dl, bool ds, int lpc = 0)
+{
+    PassShape sh{};
+    sh.map = map;
+    sh.direct_load = dl;
+    sh.direct_store = ds;
+    sh.points_per_thread = 16;
+    sh.threads_per_line = (d.n + 15) / 16;
+    sh.lines_per_cta = lpc > 0 ? lpc : smooth_line_lpc(d, map);
+    while (sh.lines_per_cta > 1 && smooth_line_smem(d, sh.lines_per_cta) > kMaxSmemBytes)
+        sh.lines_per_cta /= 2;
+    sh.smem_bytes = smooth_line_smem(d, sh.lines_per_cta);
     return sh;
 }
 
@@ -577,6 +597,11 @@ bool heuristic_shape(const PassDesc& d, PassMap map, bool dl, bool ds, PassShape
 {
     if (std::getenv("CRDFFT_PIPELINE") != nullptr && pipe_shape(d, map, out))
         return true;
+    if (smooth_pass(d))
+    {
+        *out = smooth_shape(d, map, dl, ds);
+        return true;
+    }
     const bool want32 = d.n > 8192 || (map == PassMap::Col && d.n >= 2048);
     if (want32)
     {
@@ -643,6 +668,15 @@ std::vector<PassShape> candidate_shapes(const PassDesc& d, PassMap map, bool dl,
             out.push_back(t);
         }
     };
+    if (smooth_pass(d))
+    {
+        const PassShape base = smooth_shape(d, map, dl, ds);
+        out.push_back(base);
+        for (int lpc : {base.lines_per_cta / 2, base.lines_per_cta * 2})
+            if (lpc >= 1 && lpc <= pass_lines_per_cta_limit() && smooth_line_smem(d, lpc) <= kMaxSmemBytes)
+                out.push_back(smooth_shape(d, map, dl, ds, lpc));
+        return out;
+    }
     for (int P : {16, 32})
     {
         const int T = (d.n + P - 1) / P;
@@ -674,7 +708,15 @@ bool choose_shape(const PassDesc& d, PassMap map, bool dl, bool ds, PassShape* o
     if (wisdom_lookup(key, &w))
     {
         PassShape sh;
-        if (w.pipelined ? pipe_shape(d, map, &sh, w.lines_per_cta)
+        if (smooth_pass(d) && !w.pipelined && !w.tma_store)
+        {
+            if (w.lines_per_cta >= 1 && w.lines_per_cta <= pass_lines_per_cta_limit())
+            {
+                *out = smooth_shape(d, map, dl, ds, w.lines_per_cta);
+                return true;
+            }
+        }
+        else if (w.pipelined ? pipe_shape(d, map, &sh, w.lines_per_cta)
                         : (sh = shape_with(d.n, d.nstages, map, dl, ds, w.points_per_thread, w.lines_per_cta),
                            sh.wide_regs = w.wide_regs, sh.tma_store = w.tma_store,
                            sh.threads_per_line * sh.lines_per_cta <= pass_threads_limit(sh.points_per_thread, d.n) &&
@@ -1031,9 +1073,11 @@ struct FourStepTw
     const void* lo = nullptr;
 };
 
-// The descriptor of a line pass (no launch shape yet).
+// The descriptor of a line pass (no launch shape yet). line: for the line-pass kernels, which take lengths without a
+// compile-time schedule in their own radices (smooth_radices).
 crdfft_status make_pass_desc(Plan& p, long long n, long long lines, long long lpg, LineMap in, LineMap out,
-                             bool conj_in, bool conj_out, float scale, const FourStepTw& ftw, PassDesc* out_desc)
+                             bool conj_in, bool conj_out, float scale, const FourStepTw& ftw, PassDesc* out_desc,
+                             bool line = false)
 {
     std::vector<int> rad;
     // radix-32 schedules for unit-stride passes only (the single passes); CRDFFT_R32_ROWS=1 also for passes that
@@ -1047,11 +1091,19 @@ crdfft_status make_pass_desc(Plan& p, long long n, long long lines, long long lp
     d.nstages = static_cast<int>(rad.size());
     for (size_t i = 0; i < rad.size(); ++i)
         d.radix[i] = rad[i];
+    if (line && !pass_has_static(d, 16) && !pass_has_static(d, 32))
+    {
+        if (!smooth_radices(n, rad) || static_cast<int>(rad.size()) > kMaxStages)
+            return CRDFFT_UNSUPPORTED_SIZE;
+        d.nstages = static_cast<int>(rad.size());
+        for (size_t i = 0; i < rad.size(); ++i)
+            d.radix[i] = rad[i];
+    }
     d.lines = lines;
     d.lines_per_group = lpg;
     d.in = in;
     d.out = out;
-    const crdfft_status st = twiddle_table(p, n, &d.tw, r32);
+    const crdfft_status st = twiddle_table(p, rad, &d.tw);
     if (st != CRDFFT_OK)
         return st;
     d.ftw_M = ftw.M;
@@ -1076,7 +1128,7 @@ crdfft_status make_line_step(Plan& p, long long n, long long lines, long long lp
     Step s;
     s.kind = StepKind::Line;
     PassDesc& d = s.pass;
-    const crdfft_status st = make_pass_desc(p, n, lines, lpg, in, out, conj_in, conj_out, scale, ftw, &d);
+    const crdfft_status st = make_pass_desc(p, n, lines, lpg, in, out, conj_in, conj_out, scale, ftw, &d, true);
     if (st != CRDFFT_OK)
         return st;
     // Thread map: along the elements when the loading side is unit-stride, across lines when adjacent lines are
@@ -2300,7 +2352,7 @@ crdfft_status build_uneven(Plan& p, const int64_t* sizes, int64_t count, const i
         sc.nstages = static_cast<int>(rad.size());
         for (size_t i = 0; i < rad.size(); ++i)
             sc.radix[i] = rad[i];
-        const crdfft_status st = twiddle_table(p, n, &sc.tw, false, false);
+        const crdfft_status st = twiddle_table(p, rad, &sc.tw);
         if (st != CRDFFT_OK)
             return st;
         *idx = static_cast<int>(scheds.size());

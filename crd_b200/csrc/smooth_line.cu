@@ -1,0 +1,343 @@
+// The line-FFT pass of every 7-smooth length without a compile-time schedule (240, 1000, 3000, 6144 ..): the tile code
+// of smooth_line.cuh between the pass's global line maps, with the conjugations, scale and four-step twiddle of the
+// pass in the first and last stage's accesses.
+
+#include "index.cuh"
+#include "kernels.hpp"
+#include "pass_desc.hpp"
+#include "smooth_line.cuh"
+#include "smooth_plan.hpp"
+
+#include <algorithm>
+#include <atomic>
+#include <map>
+
+namespace crdfft
+{
+
+namespace
+{
+
+// Arithmetic of one radix's butterfly a point (FP32 instructions), and what a stage costs besides (shared-memory
+// round trip, addresses, twiddle).
+struct RadixCost
+{
+    int R;
+    double per_point;
+};
+constexpr RadixCost kRadices[] = {{2, 2.0},   {3, 4.7},   {4, 4.0},   {5, 7.6},   {6, 6.7},   {7, 9.4},
+                                  {8, 6.5},   {9, 12.0},  {10, 9.6},  {12, 8.7},  {14, 11.4}, {15, 12.3},
+                                  {16, 10.5}, {18, 14.0}, {20, 11.6}, {21, 14.1}, {24, 11.7}, {25, 19.0}};
+constexpr double kStageCost = 14.0;     // a point: shared-memory round trip, twiddle
+constexpr double kButterflyCost = 25.0; // a butterfly: its indices and addresses
+// The wide build's fewer resident warps (96 registers): 720 8.10.9 67.6 us a 256 MiB batch, 240 16.15 49.5 against
+// 12.20 59.2, but 3000 12.10.25 78.8 against 10.10.6.5 97.0, a stage more.
+constexpr double kWideCost = 1.12;
+
+struct Best
+{
+    double cost = 1e30;
+    int R = 0;
+};
+
+// Cheapest product of radices up to `top` for n.
+double cheapest(long long n, int top, std::map<long long, Best>& memo)
+{
+    if (n == 1)
+        return 0.0;
+    auto it = memo.find(n);
+    if (it != memo.end())
+        return it->second.cost;
+    Best b;
+    for (const RadixCost& r : kRadices)
+        if (r.R <= top && n % r.R == 0)
+        {
+            const double c = cheapest(n / r.R, top, memo) + kStageCost + kButterflyCost / r.R + r.per_point;
+            if (c < b.cost)
+                b = Best{c, r.R};
+        }
+    memo[n] = b;
+    return b.cost;
+}
+
+} // namespace
+
+bool smooth_wide(const int* radix, int nstages)
+{
+    for (int i = 0; i < nstages; ++i)
+        if (radix[i] > 16)
+            return true;
+    return false;
+}
+
+bool smooth_radices(long long n, std::vector<int>& out)
+{
+    out.clear();
+    if (n < 1)
+        return false;
+    if (n == 1)
+        out.push_back(1);
+    std::map<long long, Best> narrow, wide;
+    const double cn = cheapest(n, 16, narrow), cw = kWideCost * cheapest(n, 25, wide);
+    std::map<long long, Best>& memo = cw < cn ? wide : narrow;
+    for (long long m = n; m > 1;)
+    {
+        const Best& b = memo[m];
+        if (b.R == 0)
+            return false;
+        out.push_back(b.R);
+        m /= b.R;
+    }
+    if (out.size() > static_cast<size_t>(kSmoothStages))
+        return false;
+    // Largest first (most loads in flight a thread, and the last stage's runs n / Rs in global memory are long), the
+    // smallest in the middle: 60 as 12.5 51.6 us against 4.15 62.6, 5000 as 25.10.20 83.2 against 10.20.25 89.1.
+    std::sort(out.rbegin(), out.rend());
+    if (out.size() > 2)
+        std::swap(out[1], out.back());
+    return true;
+}
+
+bool smooth_sched(int n, const int* radix, int nstages, const void* tw, SmoothSched* out)
+{
+    if (nstages < 1 || nstages > kSmoothStages || n > 65535)
+        return false;
+    SmoothSched s{};
+    s.n = n;
+    s.ns = nstages;
+    s.tw = tw;
+    auto magic = [](int d) { return d <= 1 ? 0u : 0xFFFFFFFFu / static_cast<unsigned>(d) + 1u; };
+    const int R1 = radix[0];
+    const int n1 = n / R1;
+    s.p1 = nstages > 1 ? n1 | 1 : n1;
+    s.m1 = magic(R1);
+    int L = 1, off = 0;
+    for (int i = 0; i < nstages; ++i)
+    {
+        SmoothStage& t = s.st[i];
+        t.R = radix[i];
+        t.L = L;
+        t.N = n / t.R;
+        t.ni = n / (L * t.R);
+        t.C = i == 0 ? t.N : t.N / R1;
+        t.tw = off;
+        t.mN = magic(t.N);
+        t.mC = magic(t.C);
+        t.mni = magic(t.ni);
+        if (L > 1)
+            off += (t.R - 1) * L;
+        L *= t.R;
+    }
+    if (L != n)
+        return false;
+    *out = s;
+    return true;
+}
+
+namespace smooth
+{
+namespace
+{
+
+struct Tile
+{
+    int lpc;
+    int sl, sp;
+    int first, mid, last; // Lanes::across of each stage
+    int flat;             // every tile's lines lie in one address group, or wrap into the next one at most once
+};
+
+// EPI: 0 plain, 1 conjugations and scale, 2 also the four-step twiddle.
+template <int EPI> struct LineIO
+{
+    const PassDesc& d;
+    const float2* gin;
+    float2* gout;
+    long long line0, g0, q0;
+    int flat;
+    float in_im, out_re, out_im;
+
+    __device__ __forceinline__ void where(int l, long long& g, long long& q) const
+    {
+        if (d.lines_per_group == 1)
+        {
+            g = line0 + l;
+            q = 0;
+        }
+        else if (flat)
+        {
+            const bool wrap = q0 + l >= d.lines_per_group;
+            g = wrap ? g0 + 1 : g0;
+            q = wrap ? q0 + l - d.lines_per_group : q0 + l;
+        }
+        else
+        {
+            g = idiv(line0 + l, d.lines_per_group);
+            q = line0 + l - g * d.lines_per_group;
+        }
+    }
+    template <int R> __device__ __forceinline__ void get(float2* v, int l, int b, int N) const
+    {
+        long long g, q;
+        where(l, g, q);
+        const float2* p = gin + g * d.in.gdist + q * d.in.ldist + static_cast<long long>(b) * d.in.estride;
+        const long long step = static_cast<long long>(N) * d.in.estride;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+        {
+            v[r] = __ldcs(p);
+            p += step;
+        }
+        if constexpr (EPI > 0)
+        {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                v[r].y *= in_im;
+        }
+    }
+    template <int R> __device__ __forceinline__ void put(float2* v, int l, int b, int N) const
+    {
+        long long g, q;
+        where(l, g, q);
+        float2* p = gout + g * d.out.gdist + q * d.out.ldist + static_cast<long long>(b) * d.out.estride;
+        const long long step = static_cast<long long>(N) * d.out.estride;
+        if constexpr (EPI == 2)
+        {
+            const int qi = static_cast<int>(idiv(q, d.ftw_div));
+            const float2* th = static_cast<const float2*>(d.ftw_hi) + (qi >> 4) * d.n + b;
+            const float2* tl = static_cast<const float2*>(d.ftw_lo) + b * 16 + (qi & 15);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                v[r] = cmul(v[r], cmul(__ldg(th + r * N), __ldg(tl + r * N * 16)));
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+        {
+            if constexpr (EPI > 0)
+                v[r] = make_float2(v[r].x * out_re, v[r].y * out_im);
+            __stcs(p, v[r]);
+            p += step;
+        }
+    }
+};
+
+template <int EPI, bool WIDE>
+__global__ void __maxnreg__(WIDE ? 96 : EPI == 2 ? 72 : 64)
+    smooth_line_kernel(const PassDesc d, const SmoothSched s, const Tile t, const float2* gin, float2* gout)
+{
+    extern __shared__ float2 sm[];
+    const long long line0 = static_cast<long long>(blockIdx.x) * t.lpc;
+    const long long left = d.lines - line0;
+    const int lines = left < t.lpc ? static_cast<int>(left) : t.lpc;
+    const long long g0 = idiv(line0, d.lines_per_group);
+    const LineIO<EPI> io{d,      gin,
+                         gout,   line0,
+                         g0,     line0 - g0 * d.lines_per_group,
+                         t.flat, d.conj_in ? -1.0f : 1.0f,
+                         d.scale, d.conj_out ? -d.scale : d.scale};
+    run_tile<WIDE>(s, sm, t.sl, t.sp, t.lpc, lines, Lanes{t.first}, Lanes{t.mid}, Lanes{t.last}, io);
+}
+
+int log2_exact(int v)
+{
+    int l = 0;
+    while ((1 << l) < v)
+        ++l;
+    return (1 << l) == v ? l : -1;
+}
+
+// The tile of a pass at `lpc` lines a CTA: layout and thread maps.
+Tile tile_of(const PassDesc& d, const SmoothSched& s, int lpc)
+{
+    Tile t{};
+    t.lpc = lpc;
+    const int places = s.st[0].R * s.p1;
+    const int lg = log2_exact(lpc);
+    const bool in_across = lg > 0 && d.in.estride != 1 && d.in.ldist == 1 && d.lines_per_group > 1;
+    const bool out_across = lg > 0 && d.out.estride != 1 && d.out.ldist == 1 && d.lines_per_group > 1;
+    // Lines interleaved when the first stage runs across them (8 bytes apart, as they arrive); else one line after
+    // another, an odd number of places apart, so that a last stage across the lines meets no bank twice.
+    t.sp = in_across ? lpc : 1;
+    t.sl = in_across ? 1 : places | 1;
+    t.first = in_across ? lg : -1;
+    t.mid = in_across ? lg : -1;
+    t.last = out_across ? lg : -1;
+    t.flat = d.lines_per_group >= lpc ? 1 : 0;
+    return t;
+}
+
+int tile_bytes(const SmoothSched& s, int lpc) { return s.ns == 1 ? 0 : lpc * (s.st[0].R * s.p1 | 1) * 8; }
+
+} // namespace
+} // namespace smooth
+
+bool smooth_line_supported(const PassDesc& d)
+{
+    SmoothSched s;
+    return smooth_sched(d.n, d.radix, d.nstages, d.tw, &s);
+}
+
+int smooth_line_smem(const PassDesc& d, int lpc)
+{
+    SmoothSched s;
+    return smooth_sched(d.n, d.radix, d.nstages, d.tw, &s) ? smooth::tile_bytes(s, lpc) : 0;
+}
+
+// Threads of a tile: as many as the registers allow the CTAs that shared memory allows, 128 to 512 (1000-point lines
+// along: 128 threads 68.8 us, 320 71.5; eight interleaved, three CTAs an SM: 320 threads 89.1 us, 416 93.2, two CTAs).
+int smooth_line_threads(const PassDesc& d, int lpc)
+{
+    const int regs = smooth_wide(d.radix, d.nstages) ? 96 : d.ftw_M != 0 ? 72 : 64;
+    const int ctas = std::max(1, 227 * 1024 / (smooth_line_smem(d, lpc) + 1024));
+    return std::clamp(65536 / regs / ctas / 32 * 32, 128, 512);
+}
+
+// Lines a CTA: along the lines, tiles of about 2200 points (many CTAs an SM hide each other's phases: 1000-point lines
+// 2 a CTA 68.8 us, 8 74.8); across them, runs of 64 bytes or more as long as a tile fits (2400 points 8 a CTA 110 us, 4
+// 114; 360 points 32 a CTA 66.3, 8 71.5).
+int smooth_line_lpc(const PassDesc& d, PassMap map)
+{
+    const bool across = map == PassMap::Col || (d.out.estride != 1 && d.out.ldist == 1 && d.lines_per_group > 1);
+    int lpc = 1;
+    if (across)
+    {
+        lpc = d.n <= 400 ? 32 : d.n <= 560 ? 16 : d.n <= 3000 ? 8 : d.n <= 6000 ? 4 : 2;
+        while (lpc < 128 && lpc * d.n < 1500)
+            lpc *= 2;
+    }
+    else
+        lpc = std::max(1, 2200 / d.n);
+    return std::min(lpc, 256);
+}
+
+cudaError_t launch_smooth_line(const PassDesc& d, int lpc, const void* in, void* out, cudaStream_t stream)
+{
+    SmoothSched s;
+    if (!smooth_sched(d.n, d.radix, d.nstages, d.tw, &s) || lpc < 1 || static_cast<long long>(lpc) * d.n > 65535)
+        return cudaErrorInvalidConfiguration;
+    const long long groups = (d.lines + lpc - 1) / lpc;
+    if (groups <= 0)
+        return cudaSuccess;
+    const int smem = smooth::tile_bytes(s, lpc);
+    if (groups > 0x7fffffffLL || smem > 227 * 1024)
+        return cudaErrorInvalidConfiguration;
+    const int epi = d.ftw_M != 0 ? 2 : (d.conj_in != 0 || d.conj_out != 0 || d.scale != 1.0f) ? 1 : 0;
+    const bool wide = smooth_wide(d.radix, d.nstages);
+    using Fn = void (*)(const PassDesc, const SmoothSched, const smooth::Tile, const float2*, float2*);
+    const Fn fns[2][3] = {{smooth::smooth_line_kernel<0, false>, smooth::smooth_line_kernel<1, false>,
+                           smooth::smooth_line_kernel<2, false>},
+                          {smooth::smooth_line_kernel<0, true>, smooth::smooth_line_kernel<1, true>,
+                           smooth::smooth_line_kernel<2, true>}};
+    const Fn fn = fns[wide ? 1 : 0][epi];
+    if (smem > 48 * 1024)
+    {
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess)
+            return e;
+    }
+    fn<<<static_cast<unsigned>(groups), smooth_line_threads(d, lpc), smem, stream>>>(
+        d, s, smooth::tile_of(d, s, lpc), static_cast<const float2*>(in), static_cast<float2*>(out));
+    return cudaGetLastError();
+}
+
+} // namespace crdfft
