@@ -23,6 +23,8 @@
 #include "chain_list.hpp"
 #include "kernels.hpp"
 #include "line_fft.cuh"
+#include "smooth_line.cuh"
+#include "smooth_plan.hpp"
 
 #include <mutex>
 
@@ -52,9 +54,18 @@ __device__ __forceinline__ bool wait_at_least(const int* p, int target, int limi
     return false;
 }
 
+// A side without a compile-time schedule runs the run-time-schedule tile (smooth_line.cuh).
+using Smooth = void;
+struct SmoothSides
+{
+    SmoothSched col_s, row_s;
+    smooth::Tile col_t, row_t;
+};
+
 template <class SC, int PC, class SR, int PR, bool REPI>
-__global__ void __maxnreg__(80) chain_fft_kernel(const ChainDesc cd, const float2* __restrict__ src,
-                                                 float2* __restrict__ dst, float2* ws)
+__global__ void __maxnreg__((std::is_void_v<SC> || std::is_void_v<SR>) ? 96 : 80)
+    chain_fft_kernel(const ChainDesc cd, const SmoothSides sides, const float2* __restrict__ src,
+                     float2* __restrict__ dst, float2* ws)
 {
     __shared__ int s_item, s_ok;
     const int tid = threadIdx.x;
@@ -93,11 +104,23 @@ __global__ void __maxnreg__(80) chain_fft_kernel(const ChainDesc cd, const float
         const long long wt = cd.batch - t0 < cd.wave_t ? cd.batch - t0 : cd.wave_t;
         float2* slot = ws + static_cast<long long>(w % cd.slots) * cd.slot_elems;
         if (is_col)
-            lfft::line_fft_tile<SC, PC, PassMap::Col, true, true, true>(cd.col, src + t0 * cd.idist, slot, idx,
-                                                                        cd.col_lpc, wt * cd.row.n, tid);
+        {
+            if constexpr (std::is_void_v<SC>)
+                smooth::pass_tile<2, true>(cd.col, sides.col_s, sides.col_t, src + t0 * cd.idist, slot, idx,
+                                           wt * cd.row.n);
+            else
+                lfft::line_fft_tile<SC, PC, PassMap::Col, true, true, true>(cd.col, src + t0 * cd.idist, slot, idx,
+                                                                            cd.col_lpc, wt * cd.row.n, tid);
+        }
         else
-            lfft::line_fft_tile<SR, PR, PassMap::Row, true, false, REPI>(cd.row, slot, dst + t0 * cd.odist, idx,
-                                                                         cd.row_lpc, wt * cd.col.n, tid);
+        {
+            if constexpr (std::is_void_v<SR>)
+                smooth::pass_tile<REPI ? 1 : 0, true>(cd.row, sides.row_s, sides.row_t, slot, dst + t0 * cd.odist,
+                                                      idx, wt * cd.col.n);
+            else
+                lfft::line_fft_tile<SR, PR, PassMap::Row, true, false, REPI>(cd.row, slot, dst + t0 * cd.odist, idx,
+                                                                             cd.row_lpc, wt * cd.col.n, tid);
+        }
     }
     // Every thread's stores of the tile are issued; one release makes them visible before the tile's signal.
     __syncthreads();
@@ -108,7 +131,7 @@ __global__ void __maxnreg__(80) chain_fft_kernel(const ChainDesc cd, const float
     }
 }
 
-using ChainFn = void (*)(const ChainDesc, const float2*, float2*, float2*);
+using ChainFn = void (*)(const ChainDesc, const SmoothSides, const float2*, float2*, float2*);
 
 template <class SC, int PC, class SR, int PR> ChainFn pick(bool repi)
 {
@@ -120,10 +143,23 @@ bool radices_are(const PassDesc& d, std::initializer_list<int> rs)
     return lfft::same_radices(d, rs);
 }
 
-// The column / row schedule pairs with a chained instance (points a thread 16 on both sides).
+bool is_static(const PassDesc& d) { return pass_has_static(d, 16) || pass_has_static(d, 32); }
+bool is_smooth(const PassDesc& d) { return !is_static(d) && smooth_line_supported(d); }
+
+// The column / row schedule pairs with a chained instance (points a thread 16 on the compile-time sides).
 ChainFn select(const PassDesc& col, const PassDesc& row)
 {
     const bool repi = lfft::pass_epi(row);
+    if (is_smooth(col))
+    {
+        if (is_smooth(row))
+            return pick<Smooth, 0, Smooth, 0>(repi);
+        if (radices_are(row, {16, 16, 4}))
+            return pick<Smooth, 0, Sched<16, 16, 4>, 16>(repi);
+        if (radices_are(row, {16, 8, 4}))
+            return pick<Smooth, 0, Sched<16, 8, 4>, 16>(repi);
+        return nullptr;
+    }
     if (radices_are(row, {16, 16, 4}))
     {
         if (radices_are(col, {7, 5, 3}))
@@ -150,13 +186,9 @@ bool chain_supported(const PassDesc& col, const PassDesc& row)
     return col.in.ldist == 1 && col.out.ldist == 1 && row.in.estride == 1 && row.ftw_M == 0 && col.ftw_M != 0;
 }
 
-int chain_smem_bytes(int n1, int n2)
+int chain_lines(const PassDesc& d, PassMap map)
 {
-    const int l1 = chain_lines_per_tile(n1);
-    const int l2 = chain_lines_per_tile(n2);
-    const int a = l1 * lfft::cta_line_pitch(n1, l1) * 8;
-    const int b = l2 * lfft::cta_line_pitch(n2, l2) * 8;
-    return a > b ? a : b;
+    return is_smooth(d) ? smooth_line_lpc(d, map) : chain_lines_per_tile(d.n);
 }
 
 cudaError_t launch_chain(const ChainDesc& cd, const void* in, void* out, void* ws, cudaStream_t stream)
@@ -164,7 +196,17 @@ cudaError_t launch_chain(const ChainDesc& cd, const void* in, void* out, void* w
     const ChainFn fn = select(cd.col, cd.row);
     if (fn == nullptr || cd.waves < 1 || cd.col_items < 1 || cd.row_items < 1 || cd.lag < 1 || cd.slots <= cd.lag)
         return cudaErrorInvalidConfiguration;
-    const int smem = chain_smem_bytes(cd.col.n, cd.row.n);
+    SmoothSides sides{};
+    auto side = [](const PassDesc& d, int lpc, SmoothSched* s, smooth::Tile* t) {
+        if (!is_smooth(d))
+            return lpc * lfft::cta_line_pitch(d.n, lpc) * 8;
+        return smooth_tile(d, lpc, s, t) ? smooth_line_smem(d, lpc) : -1;
+    };
+    const int a = side(cd.col, cd.col_lpc, &sides.col_s, &sides.col_t);
+    const int b = side(cd.row, cd.row_lpc, &sides.row_s, &sides.row_t);
+    if (a < 0 || b < 0)
+        return cudaErrorInvalidConfiguration;
+    const int smem = a > b ? a : b;
     static std::mutex mu;
     {
         std::lock_guard<std::mutex> lk(mu);
@@ -176,7 +218,7 @@ cudaError_t launch_chain(const ChainDesc& cd, const void* in, void* out, void* w
     if (total >= 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
     const long long grid = total;
-    fn<<<static_cast<unsigned>(grid), kChainThreads, smem, stream>>>(cd, static_cast<const float2*>(in),
+    fn<<<static_cast<unsigned>(grid), kChainThreads, smem, stream>>>(cd, sides, static_cast<const float2*>(in),
                                                                       static_cast<float2*>(out),
                                                                       static_cast<float2*>(ws));
     return cudaGetLastError();

@@ -204,7 +204,7 @@ struct ChainDesc
     long long slot_elems; // wave_t * n: one wave's intermediate
     int slots;            // intermediate slots (waves in flight)
     int lag;              // a wave's row tiles follow the column tiles of the wave `lag` later; 1 <= lag < slots
-    int col_lpc;          // lines a column tile (chain_lines_per_tile(n1))
+    int col_lpc;          // lines a column tile (chain_lines)
     int row_lpc;          // lines a row tile
     long long col_items;  // column tiles a wave: ceil(wave_t * n2 / col_lpc)
     long long row_items;  // row tiles a wave: ceil(wave_t * n1 / row_lpc)
@@ -212,6 +212,7 @@ struct ChainDesc
     int spin_limit;       // polls a dependency wait may take before it gives up (status word |= 1)
 };
 bool chain_supported(const PassDesc& col, const PassDesc& row);
+int chain_lines(const PassDesc& d, PassMap map); // lines a tile
 cudaError_t launch_chain(const ChainDesc& cd, const void* in, void* out, void* ws, cudaStream_t stream);
 
 // Elementwise scale of `count` complex values (used by normalisations that no pass can absorb).

@@ -252,10 +252,9 @@ bool has_static_schedule(long long n, bool use32 = false)
     return pass_has_static(d, 16) || pass_has_static(d, 32);
 }
 
-// The four-step split n = n1 * n2 (pass 1 transforms the n2 columns of length n1, pass 2 the n1 rows of length n2),
-// both halves within one CTA. Preference, in order: both halves have compile-time schedules (e.g. 107520 = 105 x
-// 1024); n2 a multiple of 16, so pass 1's column tiles stay whole; closest to square.
-bool four_step_split(long long n, long long* n1, long long* n2)
+// The split of a long column n = n1 * n2 whose halves both run as column passes (a 2-D transform's long columns), both
+// within one CTA. Preference, in order: both halves have compile-time schedules; n2 a multiple of 16; closest to square.
+bool column_split(long long n, long long* n1, long long* n2)
 {
     long long best1 = 0, best2 = 0;
     double best_score = 1e300;
@@ -285,6 +284,67 @@ bool four_step_split(long long n, long long* n1, long long* n2)
         return false;
     *n1 = best1;
     *n2 = best2;
+    return true;
+}
+
+// The four-step split n = n1 * n2 (pass 1 transforms the n2 columns of length n1, pass 2 the n1 rows of length n2),
+// both halves within one CTA: the cheapest sum of two measured costs, us for 2^24 points above a common base. They are
+// a least-squares fit to every split of 33 lengths from 10^4 to 2^22 (924 timings); picking by them is 3.5 % off
+// the fastest split on average (17 % at worst), the closest-to-square rule it replaces 10 % (26 %): 107520 as
+// 105 x 1024 160.7 us, 210 x 512 141.4; 2^17 as 256 x 512 132.1, 128 x 1024 123.0.
+double split_pass_cost(long long n, bool rows)
+{
+    struct Static
+    {
+        long long n;
+        double col, row; // rows of 512 and 1024 points leave by tensor stores
+    };
+    static const Static kStatic[] = {{16, -4.0, 0.1},   {32, 3.1, 26.0},     {64, 4.3, 1.4},      {105, 41.2, 34.9},
+                                     {128, 10.4, 2.0},
+                                     {256, 21.2, -10.2}, {512, 35.9, -8.5},   {1024, 37.3, -13.8}, {2048, 81.4, 32.0},
+                                     {4096, 99.2, 87.6}, {8192, 130.0, 130.0}, {16384, 250.0, 250.0}};
+    for (const Static& s : kStatic)
+        if (s.n == n)
+            return rows ? s.row : s.col;
+    std::vector<int> rad;
+    double arith = 0.0;
+    if (!smooth_radices(n, rad, &arith))
+        return 1e6;
+    const size_t ns = std::min<size_t>(rad.size(), 4);
+    const bool wide = smooth_wide(rad.data(), static_cast<int>(rad.size()));
+    const double lg = std::log2(static_cast<double>(n));
+    if (rows)
+    {
+        static const double kStages[5] = {0.0, -14.7, -9.7, 1.7, 34.3};
+        return kStages[ns] + 0.1 * arith + (wide ? 5.0 : 0.0) + 13.2 * std::max(0.0, lg - std::log2(1000.0)) +
+               (n % 16 == 0 ? 0.0 : 3.3) + (n % 4 == 0 ? 0.0 : 10.9); // runs of the columns' tiles off 128 and 32 bytes
+    }
+    static const double kStages[5] = {0.0, -26.3, -43.3, -52.4, -44.0};
+    return kStages[ns] + 1.16 * arith - (wide ? 2.6 : 0.0) + 11.7 * std::max(0.0, lg - std::log2(560.0));
+}
+
+bool four_step_split(long long n, long long* n1, long long* n2)
+{
+    long long best1 = 0;
+    double best_score = 1e300;
+    for (long long d = 2; d * d <= n; ++d)
+    {
+        if (n % d != 0 || !single_pass_ok(d) || !single_pass_ok(n / d))
+            continue;
+        for (const long long a : {d, n / d})
+        {
+            const double score = split_pass_cost(a, false) + split_pass_cost(n / a, true);
+            if (score < best_score)
+            {
+                best_score = score;
+                best1 = a;
+            }
+        }
+    }
+    if (best1 == 0)
+        return false;
+    *n1 = best1;
+    *n2 = n / best1;
     return true;
 }
 
@@ -976,7 +1036,12 @@ Decomp choose_decomp(const Plan& p, long long n, long long batch, long long istr
 {
     if (t_forced != nullptr && t_forced_n == n)
         return *t_forced;
-    const Decomp rule = rule_decomp(p, n, istride, idist, ostride, odist);
+    Decomp rule = rule_decomp(p, n, istride, idist, ostride, odist);
+    // The half-length transform of an R2C plan: the row pass with the fused recombination (rows of 512 or 1024 points,
+    // an even number of them) where the closest-to-square split gives one; it saves a pass over the spectrum.
+    long long c1 = 0, c2 = 0;
+    if (fused_r2c && rule.kind == 3 && column_split(n, &c1, &c2) && (c2 == 512 || c2 == 1024) && c1 % 2 == 0)
+        rule.n1 = c1;
     const std::vector<Decomp> cands = decomp_candidates(p, n, istride, idist, ostride, odist);
     {
         std::lock_guard<std::mutex> lk(g_hint_mu);
@@ -1405,21 +1470,21 @@ crdfft_status plan_c2c_1d(Plan& p, long long n, long long batch, long long istri
     {
         ChainDesc cd{};
         cd.wave_t = std::min(batch, std::max(1LL, chain_wave_bytes() / (n * 8)));
-        const int l1 = chain_lines_per_tile(static_cast<int>(n1));
-        const int l2 = chain_lines_per_tile(static_cast<int>(n2));
         FourStepTw ftw;
         ftw.M = n;
         ftw.hi = hi;
         ftw.lo = lo;
         st = make_pass_desc(p, n1, cd.wave_t * n2, n2, LineMap{idist, 1, n2}, LineMap{n, 1, n2}, conj_in, false,
-                            1.0f, ftw, &cd.col);
+                            1.0f, ftw, &cd.col, true);
         if (st != CRDFFT_OK)
             return st;
         st = make_pass_desc(p, n2, cd.wave_t * n1, n1, LineMap{n, n2, 1}, LineMap{odist, ostride, n1 * ostride}, false,
-                            conj_out, scale, FourStepTw{}, &cd.row);
+                            conj_out, scale, FourStepTw{}, &cd.row, true);
         if (st != CRDFFT_OK)
             return st;
         cd.row.discard_in = l2_discard() ? 1 : 0;
+        const int l1 = chain_lines(cd.col, PassMap::Col);
+        const int l2 = chain_lines(cd.row, PassMap::Row);
         if (l1 >= 1 && l2 >= 1 && l1 <= pass_lines_per_cta_limit() && l2 <= pass_lines_per_cta_limit() &&
             chain_supported(cd.col, cd.row))
         {
@@ -1934,7 +1999,7 @@ crdfft_status build_nd(Plan& p)
     long long cn1 = 0, cn2 = 0;
     const bool split_cols = rank == 2 && d.dims[0] >= 2048 && d.dims[1] >= 16 && idist == total && odist == total &&
                             d.batch <= 8 && std::getenv("CRDFFT_NO_SPLIT_COLUMNS") == nullptr &&
-                            four_step_split(d.dims[0], &cn1, &cn2) && single_pass_ok(d.dims[1]);
+                            column_split(d.dims[0], &cn1, &cn2) && single_pass_ok(d.dims[1]);
     if (split_cols)
     {
         const long long rows = d.dims[0], cols = d.dims[1];

@@ -70,7 +70,7 @@ bool smooth_wide(const int* radix, int nstages)
     return false;
 }
 
-bool smooth_radices(long long n, std::vector<int>& out)
+bool smooth_radices(long long n, std::vector<int>& out, double* arith)
 {
     out.clear();
     if (n < 1)
@@ -80,6 +80,8 @@ bool smooth_radices(long long n, std::vector<int>& out)
     std::map<long long, Best> narrow, wide;
     const double cn = cheapest(n, 16, narrow), cw = kWideCost * cheapest(n, 25, wide);
     std::map<long long, Best>& memo = cw < cn ? wide : narrow;
+    if (arith != nullptr)
+        *arith = std::min(cn, cw);
     for (long long m = n; m > 1;)
     {
         const Best& b = memo[m];
@@ -139,103 +141,11 @@ namespace smooth
 namespace
 {
 
-struct Tile
-{
-    int lpc;
-    int sl, sp;
-    int first, mid, last; // Lanes::across of each stage
-    int flat;             // every tile's lines lie in one address group, or wrap into the next one at most once
-};
-
-// EPI: 0 plain, 1 conjugations and scale, 2 also the four-step twiddle.
-template <int EPI> struct LineIO
-{
-    const PassDesc& d;
-    const float2* gin;
-    float2* gout;
-    long long line0, g0, q0;
-    int flat;
-    float in_im, out_re, out_im;
-
-    __device__ __forceinline__ void where(int l, long long& g, long long& q) const
-    {
-        if (d.lines_per_group == 1)
-        {
-            g = line0 + l;
-            q = 0;
-        }
-        else if (flat)
-        {
-            const bool wrap = q0 + l >= d.lines_per_group;
-            g = wrap ? g0 + 1 : g0;
-            q = wrap ? q0 + l - d.lines_per_group : q0 + l;
-        }
-        else
-        {
-            g = idiv(line0 + l, d.lines_per_group);
-            q = line0 + l - g * d.lines_per_group;
-        }
-    }
-    template <int R> __device__ __forceinline__ void get(float2* v, int l, int b, int N) const
-    {
-        long long g, q;
-        where(l, g, q);
-        const float2* p = gin + g * d.in.gdist + q * d.in.ldist + static_cast<long long>(b) * d.in.estride;
-        const long long step = static_cast<long long>(N) * d.in.estride;
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-        {
-            v[r] = __ldcs(p);
-            p += step;
-        }
-        if constexpr (EPI > 0)
-        {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                v[r].y *= in_im;
-        }
-    }
-    template <int R> __device__ __forceinline__ void put(float2* v, int l, int b, int N) const
-    {
-        long long g, q;
-        where(l, g, q);
-        float2* p = gout + g * d.out.gdist + q * d.out.ldist + static_cast<long long>(b) * d.out.estride;
-        const long long step = static_cast<long long>(N) * d.out.estride;
-        if constexpr (EPI == 2)
-        {
-            const int qi = static_cast<int>(idiv(q, d.ftw_div));
-            const float2* th = static_cast<const float2*>(d.ftw_hi) + (qi >> 4) * d.n + b;
-            const float2* tl = static_cast<const float2*>(d.ftw_lo) + b * 16 + (qi & 15);
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                v[r] = cmul(v[r], cmul(__ldg(th + r * N), __ldg(tl + r * N * 16)));
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-        {
-            if constexpr (EPI > 0)
-                v[r] = make_float2(v[r].x * out_re, v[r].y * out_im);
-            __stcs(p, v[r]);
-            p += step;
-        }
-    }
-};
-
 template <int EPI, bool WIDE>
 __global__ void __maxnreg__(WIDE ? 96 : EPI == 2 ? 72 : 64)
     smooth_line_kernel(const PassDesc d, const SmoothSched s, const Tile t, const float2* gin, float2* gout)
 {
-    extern __shared__ float2 sm[];
-    const long long line0 = static_cast<long long>(blockIdx.x) * t.lpc;
-    const long long left = d.lines - line0;
-    const int lines = left < t.lpc ? static_cast<int>(left) : t.lpc;
-    const long long g0 = idiv(line0, d.lines_per_group);
-    const LineIO<EPI> io{d,      gin,
-                         gout,   line0,
-                         g0,     line0 - g0 * d.lines_per_group,
-                         t.flat, d.conj_in ? -1.0f : 1.0f,
-                         d.scale, d.conj_out ? -d.scale : d.scale};
-    run_tile<WIDE>(s, sm, t.sl, t.sp, t.lpc, lines, Lanes{t.first}, Lanes{t.mid}, Lanes{t.last}, io);
+    pass_tile<EPI, WIDE>(d, s, t, gin, gout, blockIdx.x, d.lines);
 }
 
 int log2_exact(int v)
@@ -281,6 +191,14 @@ int smooth_line_smem(const PassDesc& d, int lpc)
 {
     SmoothSched s;
     return smooth_sched(d.n, d.radix, d.nstages, d.tw, &s) ? smooth::tile_bytes(s, lpc) : 0;
+}
+
+bool smooth_tile(const PassDesc& d, int lpc, SmoothSched* s, smooth::Tile* t)
+{
+    if (!smooth_sched(d.n, d.radix, d.nstages, d.tw, s) || lpc < 1 || static_cast<long long>(lpc) * d.n > 65535)
+        return false;
+    *t = smooth::tile_of(d, *s, lpc);
+    return true;
 }
 
 // Threads of a tile: as many as the registers allow the CTAs that shared memory allows, 128 to 512 (1000-point lines

@@ -19,6 +19,8 @@
 // strided reads start on odd multiples of the bank width.
 
 #include "codelets.cuh"
+#include "index.cuh"
+#include "pass_desc.hpp"
 
 #include <cuda_runtime.h>
 
@@ -56,6 +58,16 @@ struct SmoothSched
 
 namespace smooth
 {
+
+// A tile of a line pass: lines a CTA, the places' strides, the thread map of each stage.
+struct Tile
+{
+    int lpc;
+    int sl, sp;
+    int first, mid, last; // Lanes::across of each stage
+    int flat;             // every tile's lines lie in one address group, or wrap into the next one at most once
+};
+
 namespace
 {
 
@@ -277,6 +289,111 @@ __device__ __forceinline__ void run_tile(const SmoothSched& s, float2* sm, int s
     {
         __syncthreads();
         with_radix<WIDE>(s.st[s.ns - 1].R, [&]<int R>() { last_stage<R>(s, last, sm, sl, sp, lpc, lines, io); });
+    }
+}
+
+// ---- a line pass (pass_desc.hpp) as the tile's input and output ---------------------------------------------------
+
+// EPI: 0 plain, 1 conjugations and scale, 2 also the four-step twiddle.
+template <int EPI> struct LineIO
+{
+    const PassDesc& d;
+    const float2* gin;
+    float2* gout;
+    long long line0, g0, q0;
+    int flat;
+    float in_im, out_re, out_im;
+
+    __device__ __forceinline__ void where(int l, long long& g, long long& q) const
+    {
+        if (d.lines_per_group == 1)
+        {
+            g = line0 + l;
+            q = 0;
+        }
+        else if (flat)
+        {
+            const bool wrap = q0 + l >= d.lines_per_group;
+            g = wrap ? g0 + 1 : g0;
+            q = wrap ? q0 + l - d.lines_per_group : q0 + l;
+        }
+        else
+        {
+            g = idiv(line0 + l, d.lines_per_group);
+            q = line0 + l - g * d.lines_per_group;
+        }
+    }
+    template <int R> __device__ __forceinline__ void get(float2* v, int l, int b, int N) const
+    {
+        long long g, q;
+        where(l, g, q);
+        const float2* p = gin + g * d.in.gdist + q * d.in.ldist + static_cast<long long>(b) * d.in.estride;
+        const long long step = static_cast<long long>(N) * d.in.estride;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+        {
+            v[r] = __ldcs(p);
+            p += step;
+        }
+        if constexpr (EPI > 0)
+        {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                v[r].y *= in_im;
+        }
+    }
+    template <int R> __device__ __forceinline__ void put(float2* v, int l, int b, int N) const
+    {
+        long long g, q;
+        where(l, g, q);
+        float2* p = gout + g * d.out.gdist + q * d.out.ldist + static_cast<long long>(b) * d.out.estride;
+        const long long step = static_cast<long long>(N) * d.out.estride;
+        if constexpr (EPI == 2)
+        {
+            const int qi = static_cast<int>(idiv(q, d.ftw_div));
+            const float2* th = static_cast<const float2*>(d.ftw_hi) + (qi >> 4) * d.n + b;
+            const float2* tl = static_cast<const float2*>(d.ftw_lo) + b * 16 + (qi & 15);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                v[r] = cmul(v[r], cmul(__ldg(th + r * N), __ldg(tl + r * N * 16)));
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+        {
+            if constexpr (EPI > 0)
+                v[r] = make_float2(v[r].x * out_re, v[r].y * out_im);
+            __stcs(p, v[r]);
+            p += step;
+        }
+    }
+};
+
+// Tile `blk` of a pass of `nlines` lines: lines [blk * lpc, blk * lpc + lpc).
+template <int EPI, bool WIDE>
+__device__ __forceinline__ void pass_tile(const PassDesc& d, const SmoothSched& s, const Tile& t, const float2* gin,
+                                          float2* gout, long long blk, long long nlines)
+{
+    extern __shared__ float2 sm[];
+    const long long line0 = blk * t.lpc;
+    const long long left = nlines - line0;
+    const int lines = left < t.lpc ? static_cast<int>(left) : t.lpc;
+    const long long g0 = idiv(line0, d.lines_per_group);
+    const LineIO<EPI> io{d,      gin,
+                         gout,   line0,
+                         g0,     line0 - g0 * d.lines_per_group,
+                         t.flat, d.conj_in ? -1.0f : 1.0f,
+                         d.scale, d.conj_out ? -d.scale : d.scale};
+    run_tile<WIDE>(s, sm, t.sl, t.sp, t.lpc, lines, Lanes{t.first}, Lanes{t.mid}, Lanes{t.last}, io);
+    if (d.discard_in && s.ns > 1 && d.in.estride == 1 && d.in.ldist == d.n && d.in.gdist == d.lines_per_group * d.n)
+    {
+        // A dead input (a four-step intermediate in L2; the barriers since the first stage end this CTA's reads of
+        // it): drop the 128-byte lines that lie wholly in the tile, whose rows are consecutive in memory, so that L2
+        // does not write them back. A line shared with the next tile stays: that CTA may not have read it yet.
+        const uintptr_t lo = reinterpret_cast<uintptr_t>(gin + line0 * d.n);
+        const uintptr_t hi = lo + static_cast<uintptr_t>(lines) * d.n * 8;
+        for (uintptr_t p = ((lo + 127) & ~static_cast<uintptr_t>(127)) + threadIdx.x * 128; p + 128 <= hi;
+             p += blockDim.x * 128)
+            asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory");
     }
 }
 
