@@ -121,23 +121,33 @@ struct RealRecombine
 cudaError_t launch_r2c_post(const RealRecombine& p, const void* z, void* out, cudaStream_t stream);
 cudaError_t launch_c2r_pre(const RealRecombine& p, const void* in, void* z, cudaStream_t stream);
 
-// Bluestein helpers (real_ops.cu): chirp pre-multiply with zero padding, pointwise spectrum product, chirp
-// post-multiply. The math of include/crd/hesap/fft/bluestein.hpp:87-136.
+// Bluestein (chirp_fft.cu), the math of include/crd/hesap/fft/bluestein.hpp:87-136: the chirp product with zero
+// padding to m, the circular convolution with the chirp of length m and the chirp product on the way out, as one
+// launch (chirp_line, m in one CTA: n1 = 0) or three over a four-step m = n1 n2 (columns in, rows, columns out).
 struct ChirpDesc
 {
-    long long n;      // transform length
-    long long m;      // padded power-of-two length (>= 2n - 1)
-    long long batch;
-    long long xdist;  // distance between transforms on the n side
-    long long wdist;  // distance between transforms on the m side (scratch)
+    long long n;       // transform length
+    long long m;       // padded 7-smooth length (>= 2n - 1)
+    long long n1, n2;  // its four-step split; 0, 0: one CTA a line
+    long long batch;   // transforms of this launch
+    long long idist;   // distance between transforms, input and output
+    long long odist;
     const void* chirp; // float2 exp(+iπ k²/n), k < n
-    const void* bfft;  // float2 FFT_m(b_circ), length m
+    const void* bfft;  // float2 FFT_m(b_circ): frequency k; with a split, frequency k1 + n1 k2 at k1 n2 + k2
+    const void* hi;    // four-step twiddles of m = n1 n2 (PassDesc::ftw_hi, ftw_lo)
+    const void* lo;
+    const void* tw1;   // stage twiddles of the column length (or of m) and of the row length
+    const void* tw2;
     int conj;          // inverse direction: conjugate x on the way in and the result on the way out
     float scale;       // final scale (1/m, times 1/n for the normalised inverse)
 };
-cudaError_t launch_chirp_pre(const ChirpDesc& p, const void* x, void* w, cudaStream_t stream);
-cudaError_t launch_spectrum_mul(const ChirpDesc& p, void* w, cudaStream_t stream);
-cudaError_t launch_chirp_post(const ChirpDesc& p, const void* w, void* x, cudaStream_t stream);
+// The longest m one CTA transforms (two CTAs an SM); the radices of a convolution length (two or more stages), false when none.
+constexpr long long kChirpLine = 14000;
+bool chirp_radices(long long m, std::vector<int>& out, double* arith = nullptr);
+cudaError_t launch_chirp_line(const ChirpDesc& p, const void* x, void* out, cudaStream_t stream);
+cudaError_t launch_chirp_cols_in(const ChirpDesc& p, const void* x, void* w, cudaStream_t stream);
+cudaError_t launch_chirp_rows(const ChirpDesc& p, void* w, cudaStream_t stream);
+cudaError_t launch_chirp_cols_out(const ChirpDesc& p, const void* w, void* out, cudaStream_t stream);
 
 // Cluster-fused four-step (cluster_fft.cu): one thread-block cluster per transform of n = a.n * b.n, columns of
 // length a.n (descriptor a: in.estride = b.n, stage twiddles, four-step twiddle tables), rows of length b.n

@@ -107,9 +107,10 @@ enum class StepKind : int
     Zero,
     R2CPost,
     C2RPre,
-    ChirpPre,
-    SpecMul,
-    ChirpPost,
+    ChirpLine,
+    ChirpColsIn,
+    ChirpRows,
+    ChirpColsOut,
     Scale,
     Chain
 };
@@ -292,7 +293,10 @@ bool column_split(long long n, long long* n1, long long* n2)
 // a least-squares fit to every split of 33 lengths from 10^4 to 2^22 (924 timings); picking by them is 3.5 % off
 // the fastest split on average (17 % at worst), the closest-to-square rule it replaces 10 % (26 %): 107520 as
 // 105 x 1024 160.7 us, 210 x 512 141.4; 2^17 as 256 x 512 132.1, 128 x 1024 123.0.
-double split_pass_cost(long long n, bool rows)
+// compiled: lengths with a compile-time schedule run it (the chirp convolution's passes never do).
+double split_pass_cost(long long n, bool rows, bool compiled);
+
+double split_pass_cost_of(long long n, bool rows, bool compiled)
 {
     struct Static
     {
@@ -304,7 +308,7 @@ double split_pass_cost(long long n, bool rows)
                                      {256, 21.2, -10.2}, {512, 35.9, -8.5},   {1024, 37.3, -13.8}, {2048, 81.4, 32.0},
                                      {4096, 99.2, 87.6}, {8192, 130.0, 130.0}, {16384, 250.0, 250.0}};
     for (const Static& s : kStatic)
-        if (s.n == n)
+        if (compiled && s.n == n)
             return rows ? s.row : s.col;
     std::vector<int> rad;
     double arith = 0.0;
@@ -323,17 +327,27 @@ double split_pass_cost(long long n, bool rows)
     return kStages[ns] + 1.16 * arith - (wide ? 2.6 : 0.0) + 11.7 * std::max(0.0, lg - std::log2(560.0));
 }
 
-bool four_step_split(long long n, long long* n1, long long* n2)
+double split_pass_cost(long long n, bool rows, bool compiled)
+{
+    thread_local std::map<long long, double> memo; // at most a few hundred line lengths
+    const long long key = n * 4 + (rows ? 2 : 0) + (compiled ? 1 : 0);
+    auto it = memo.find(key);
+    if (it == memo.end())
+        it = memo.emplace(key, split_pass_cost_of(n, rows, compiled)).first;
+    return it->second;
+}
+
+bool four_step_split(long long n, long long* n1, long long* n2, bool compiled = true, double* cost = nullptr)
 {
     long long best1 = 0;
     double best_score = 1e300;
-    for (long long d = 2; d * d <= n; ++d)
+    for (long long d = compiled ? 2 : 4; d * d <= n; ++d)
     {
         if (n % d != 0 || !single_pass_ok(d) || !single_pass_ok(n / d))
             continue;
         for (const long long a : {d, n / d})
         {
-            const double score = split_pass_cost(a, false) + split_pass_cost(n / a, true);
+            const double score = split_pass_cost(a, false, compiled) + split_pass_cost(n / a, true, compiled);
             if (score < best_score)
             {
                 best_score = score;
@@ -345,7 +359,58 @@ bool four_step_split(long long n, long long* n1, long long* n2)
         return false;
     *n1 = best1;
     *n2 = n / best1;
+    if (cost != nullptr)
+        *cost = best_score;
     return true;
+}
+
+// The convolution length of Bluestein's transform of n points and its four-step split (0, 0: one CTA a line): among
+// the 7-smooth m from 2n - 1 to 30 % above and the next power of two, the cheapest by the line schedules' cost rule, or
+// by the four-step passes' (us above 123 for 2^24 points) where a line does not fit one CTA.
+bool chirp_length(long long n, long long* m, long long* n1, long long* n2)
+{
+    const long long lo = std::max(2 * n - 1, 32LL);
+    long long pow2 = 1;
+    while (pow2 < lo)
+        pow2 <<= 1;
+    const long long hi = std::min(pow2, lo + lo / 10 * 3 + 8);
+    std::vector<long long> cands{pow2};
+    for (long long p7 = 1; p7 <= hi; p7 *= 7)
+        for (long long p5 = p7; p5 <= hi; p5 *= 5)
+            for (long long p3 = p5; p3 <= hi; p3 *= 3)
+                for (long long p2 = p3; p2 <= hi; p2 *= 2)
+                    if (p2 >= lo && p2 != pow2)
+                        cands.push_back(p2);
+    std::sort(cands.begin(), cands.end());
+    double best = 1e300;
+    std::vector<int> rad;
+    for (size_t i = 0; i < cands.size(); ++i)
+    {
+        const long long c = cands[i];
+        if (i > 24 && c != pow2) // the shortest ones, and the power of two
+            continue;
+        double cost = 0.0;
+        long long a = 0, b = 0;
+        if (c <= kChirpLine)
+        {
+            if (!chirp_radices(c, rad, &cost))
+                continue;
+        }
+        else if (lo <= kChirpLine || !four_step_split(c, &a, &b, false, &cost) || !chirp_radices(a, rad) ||
+                 !chirp_radices(b, rad))
+            continue;
+        else
+            cost += 123.0;
+        cost *= static_cast<double>(c);
+        if (cost < best)
+        {
+            best = cost;
+            *m = c;
+            *n1 = a;
+            *n2 = b;
+        }
+    }
+    return best < 1e300;
 }
 
 struct Plan
@@ -1577,6 +1642,84 @@ crdfft_status plan_c2c_1d(Plan& p, long long n, long long batch, long long istri
     return CRDFFT_OK;
 }
 
+// In-place FP64 transform of a 7-smooth length, for tables (Stockham, one prime a stage).
+void host_fft(std::vector<std::complex<double>>& a)
+{
+    const long long n = static_cast<long long>(a.size());
+    // W_n^k: the octant the symmetries of the circle do not give, and the rest from it where n allows
+    std::vector<std::complex<double>> w(static_cast<size_t>(n));
+    const long long direct = n % 8 == 0 ? n / 8 : n - 1;
+    for (long long k = 0; k <= direct && k < n; ++k)
+    {
+        double re, im;
+        root(k, n, &re, &im);
+        w[static_cast<size_t>(k)] = {re, im};
+    }
+    for (long long k = direct + 1; k < n; ++k)
+    {
+        const long long q = n / 4;
+        const size_t at = static_cast<size_t>(k);
+        if (k <= q) // W^{q-j} = -i conj(W^j)
+        {
+            const std::complex<double> z = w[static_cast<size_t>(q - k)];
+            w[at] = {-z.imag(), -z.real()};
+        }
+        else // W^{q+j} = -i W^j
+        {
+            const std::complex<double> z = w[static_cast<size_t>(k - q)];
+            w[at] = {z.imag(), -z.real()};
+        }
+    }
+    using cd = std::complex<double>;
+    auto mul = [](const cd& x, const cd& t) {
+        return cd(x.real() * t.real() - x.imag() * t.imag(), x.real() * t.imag() + x.imag() * t.real());
+    };
+    std::vector<cd> b(a.size());
+    long long L = 1;
+    for (long long left = n; left > 1;)
+    {
+        const int p = left % 4 == 0 ? 4 : left % 2 == 0 ? 2 : left % 3 == 0 ? 3 : left % 5 == 0 ? 5 : 7;
+        const long long nb = n / p, step = n / (L * p), turn = n / p;
+        for (long long q = 0; q < nb / L; ++q)
+            for (long long k = 0; k < L; ++k)
+            {
+                const cd* x = a.data() + q * L + k;
+                cd* y = b.data() + q * L * p + k;
+                cd v[7];
+                v[0] = x[0];
+                for (int r = 1; r < p; ++r)
+                    v[r] = L == 1 ? x[r * nb] : mul(x[r * nb], w[static_cast<size_t>(r * k * step)]);
+                if (p == 4)
+                {
+                    const cd s0 = v[0] + v[2], d0 = v[0] - v[2], s1 = v[1] + v[3], d1 = v[1] - v[3];
+                    y[0] = s0 + s1;
+                    y[L] = cd(d0.real() + d1.imag(), d0.imag() - d1.real());
+                    y[2 * L] = s0 - s1;
+                    y[3 * L] = cd(d0.real() - d1.imag(), d0.imag() + d1.real());
+                }
+                else if (p == 2)
+                {
+                    y[0] = v[0] + v[1];
+                    y[L] = v[0] - v[1];
+                }
+                else
+                    for (int o = 0; o < p; ++o)
+                    {
+                        cd z = v[0];
+                        for (int r = 1; r < p; ++r)
+                            z += mul(v[r], w[static_cast<size_t>((r * o) % p * turn)]);
+                        y[o * L] = z;
+                    }
+            }
+        a.swap(b);
+        L *= p;
+        left /= p;
+    }
+}
+
+// A wave of padded sequences of Bluestein's three-launch form (they stay in L2 between its launches).
+constexpr long long kChirpWaveBytes = 64LL << 20;
+
 crdfft_status build_c2c_rank1(Plan& p)
 {
     const crdfft_desc& d = p.desc;
@@ -1615,13 +1758,34 @@ crdfft_status build_c2c_rank1(Plan& p)
         }
         return CRDFFT_OK;
     }
-    // Bluestein: m = smallest power of two >= 2n - 1 (bluestein.hpp:36-41).
-    long long m = 1;
-    while (m < 2 * n - 1)
-        m <<= 1;
+    // Bluestein (chirp_fft.cu): a circular convolution of 7-smooth length m >= 2n - 1 (bluestein.hpp:36-41 takes the
+    // next power of two).
+    if (istride != 1 || ostride != 1)
+        return CRDFFT_UNSUPPORTED_SIZE;
+    long long m = 0, n1 = 0, n2 = 0;
+    if (!chirp_length(n, &m, &n1, &n2))
+        return CRDFFT_UNSUPPORTED_SIZE;
+    const long long B = d.batch;
+    // The three-launch form works in waves whose padded sequences stay in L2.
+    const long long wave_cap = t_arena != nullptr ? static_cast<long long>(t_arena->size / 2) : kChirpWaveBytes;
+    const long long waves = n1 == 0 ? 1 : std::max(1LL, (B * m * 8 + wave_cap - 1) / wave_cap);
+    const long long wave = std::min(B, (B + waves - 1) / waves);
+    if (t_arena != nullptr)
+    {
+        // What the fixed array serves is documented by the next power of two: its padded sequences, their spectrum
+        // and the transforms' intermediate.
+        long long p2 = 1;
+        while (p2 < 2 * n - 1)
+            p2 <<= 1;
+        const long long inner = single_pass_ok(p2) || p2 == 65536
+                                    ? 0
+                                    : std::min(B, std::max(1LL, static_cast<long long>(t_arena->size / 2) / (p2 * 8)));
+        if ((n + p2 * (1 + B + inner)) * 8 > static_cast<long long>(t_arena->size))
+            return CRDFFT_OOM;
+    }
     // chirp_k = exp(+iπ k²/n), k² reduced mod 2n (bluestein.hpp:47-53)
     std::vector<float> chirp(static_cast<size_t>(2 * n));
-    std::vector<std::complex<double>> bcirc(static_cast<size_t>(m), {0.0, 0.0});
+    std::vector<std::complex<double>> bf(static_cast<size_t>(m), {0.0, 0.0});
     for (long long k = 0; k < n; ++k)
     {
         const long long kk = static_cast<long long>((static_cast<unsigned __int128>(k) * k) % (2 * n));
@@ -1631,112 +1795,85 @@ crdfft_status build_c2c_rank1(Plan& p)
         chirp[2 * k] = static_cast<float>(re);
         chirp[2 * k + 1] = static_cast<float>(-im);
         const std::complex<double> c(re, -im);
-        bcirc[static_cast<size_t>(k)] = c;
+        bf[static_cast<size_t>(k)] = c;
         if (k > 0)
-            bcirc[static_cast<size_t>(m - k)] = c;
+            bf[static_cast<size_t>(m - k)] = c;
     }
     // FFT_m(b_circ) in FP64 on the host (the reference runs its f32 plan on the narrowed chirp; an FP64 spectrum
     // narrowed once is at least as accurate).
-    std::vector<std::complex<double>> bf(static_cast<size_t>(m));
-    {
-        // iterative radix-2 DIT in FP64
-        std::vector<std::complex<double>> a = bcirc;
-        int lg = 0;
-        while ((1LL << lg) < m)
-            ++lg;
-        for (long long i = 0; i < m; ++i)
-        {
-            long long r = 0;
-            for (int b = 0; b < lg; ++b)
-                if (i & (1LL << b))
-                    r |= 1LL << (lg - 1 - b);
-            if (i < r)
-                std::swap(a[static_cast<size_t>(i)], a[static_cast<size_t>(r)]);
-        }
-        for (long long len = 2; len <= m; len <<= 1)
-        {
-            for (long long k = 0; k < len / 2; ++k)
-            {
-                double wr, wi;
-                root(k * (m / len), m, &wr, &wi);
-                const std::complex<double> w(wr, wi);
-                for (long long s = 0; s < m; s += len)
-                {
-                    const std::complex<double> u = a[static_cast<size_t>(s + k)];
-                    const std::complex<double> v = a[static_cast<size_t>(s + k + len / 2)] * w;
-                    a[static_cast<size_t>(s + k)] = u + v;
-                    a[static_cast<size_t>(s + k + len / 2)] = u - v;
-                }
-            }
-        }
-        bf = a;
-    }
+    host_fft(bf);
     std::vector<float> bff(static_cast<size_t>(2 * m));
-    for (long long k = 0; k < m; ++k)
+    const long long rows = n1 == 0 ? 1 : n1, cols = m / rows;
+    for (long long k1 = 0; k1 < rows; ++k1) // the rows' order: frequency k1 + n1 k2 at k1 n2 + k2
+        for (long long k2 = 0; k2 < cols; ++k2)
+        {
+            const std::complex<double>& h = bf[static_cast<size_t>(k1 + rows * k2)];
+            const size_t at = static_cast<size_t>(k1 * cols + k2);
+            bff[2 * at] = static_cast<float>(h.real());
+            bff[2 * at + 1] = static_cast<float>(h.imag());
+        }
+    ChirpDesc c{};
+    c.n = n;
+    c.m = m;
+    c.n1 = n1;
+    c.n2 = n2;
+    c.idist = idist;
+    c.odist = odist;
+    void* dev = nullptr;
+    crdfft_status st = upload_table(p, chirp, &dev);
+    if (st != CRDFFT_OK)
+        return st;
+    c.chirp = dev;
+    st = upload_table(p, bff, &dev);
+    if (st != CRDFFT_OK)
+        return st;
+    c.bfft = dev;
+    std::vector<int> rad;
+    if (!chirp_radices(n1 == 0 ? m : n1, rad))
+        return CRDFFT_UNSUPPORTED_SIZE;
+    st = twiddle_table(p, rad, &c.tw1);
+    if (st != CRDFFT_OK)
+        return st;
+    if (n1 != 0)
     {
-        bff[static_cast<size_t>(2 * k)] = static_cast<float>(bf[static_cast<size_t>(k)].real());
-        bff[static_cast<size_t>(2 * k + 1)] = static_cast<float>(bf[static_cast<size_t>(k)].imag());
+        if (!chirp_radices(n2, rad))
+            return CRDFFT_UNSUPPORTED_SIZE;
+        st = twiddle_table(p, rad, &c.tw2);
+        if (st == CRDFFT_OK)
+            st = four_step_tables(p, m, n1, n2, &c.hi, &c.lo);
+        if (st != CRDFFT_OK)
+            return st;
     }
-    void* dchirp = nullptr;
-    void* dbf = nullptr;
-    crdfft_status st = upload_table(p, chirp, &dchirp);
-    if (st != CRDFFT_OK)
-        return st;
-    st = upload_table(p, bff, &dbf);
-    if (st != CRDFFT_OK)
-        return st;
-    const long long B = d.batch;
-    const long long conv = B * m; // the padded sequences live at the start of the workspace
-    long long inner_f = 0, inner_i = 0;
     for (int dir = 0; dir < 2; ++dir)
     {
-        std::vector<Step>& steps = p.steps[dir];
-        ChirpDesc c{};
-        c.n = n;
-        c.m = m;
-        c.batch = B;
-        c.wdist = m;
-        c.chirp = dchirp;
-        c.bfft = dbf;
         c.conj = dir;
-        Step pre;
-        pre.kind = StepKind::ChirpPre;
-        pre.chirp = c;
-        pre.chirp.xdist = idist;
-        pre.src = BufRef{Buf::In, 0};
-        pre.dst = BufRef{Buf::Ws, 0};
-        if (istride != 1 || ostride != 1)
-            return CRDFFT_UNSUPPORTED_SIZE;
-        steps.push_back(pre);
-        long long need = 0;
-        st = plan_c2c_1d(p, m, B, 1, m, 1, m, BufRef{Buf::Ws, 0}, BufRef{Buf::Ws, 0}, false, false, 1.0f, conv,
-                         steps, &need);
-        if (st != CRDFFT_OK)
-            return st;
-        inner_f = std::max(inner_f, need);
-        Step mul;
-        mul.kind = StepKind::SpecMul;
-        mul.chirp = c;
-        mul.dst = BufRef{Buf::Ws, 0};
-        steps.push_back(mul);
-        st = plan_c2c_1d(p, m, B, 1, m, 1, m, BufRef{Buf::Ws, 0}, BufRef{Buf::Ws, 0}, true, true, 1.0f, conv,
-                         steps, &need);
-        if (st != CRDFFT_OK)
-            return st;
-        inner_i = std::max(inner_i, need);
-        Step post;
-        post.kind = StepKind::ChirpPost;
-        post.chirp = c;
-        post.chirp.xdist = odist;
         double sc = 1.0 / static_cast<double>(m);
         if (dir == 1 && d.norm == CRDFFT_NORM_INVERSE)
             sc /= static_cast<double>(n);
-        post.chirp.scale = static_cast<float>(sc);
-        post.src = BufRef{Buf::Ws, 0};
-        post.dst = BufRef{Buf::Out, 0};
-        steps.push_back(post);
+        c.scale = static_cast<float>(sc);
+        for (long long t0 = 0; t0 < B; t0 += wave)
+        {
+            c.batch = std::min(wave, B - t0);
+            const BufRef in{Buf::In, t0 * idist}, out{Buf::Out, t0 * odist}, ws{Buf::Ws, 0};
+            auto add = [&](StepKind kind, BufRef src, BufRef dst) {
+                Step s;
+                s.kind = kind;
+                s.chirp = c;
+                s.src = src;
+                s.dst = dst;
+                p.steps[dir].push_back(s);
+            };
+            if (n1 == 0)
+                add(StepKind::ChirpLine, in, out);
+            else
+            {
+                add(StepKind::ChirpColsIn, in, ws);
+                add(StepKind::ChirpRows, ws, ws);
+                add(StepKind::ChirpColsOut, ws, out);
+            }
+        }
     }
-    p.ws_bytes = static_cast<size_t>(conv + std::max(inner_f, inner_i)) * 8;
+    p.ws_bytes = n1 == 0 ? 0 : static_cast<size_t>(wave * m) * 8;
     p.algorithm = "bluestein";
     p.factors = {n, m};
     return CRDFFT_OK;
@@ -2987,9 +3124,10 @@ crdfft_status run(Plan& p, const void* in, void* out, int dir, cudaStream_t stre
                 break;
             case StepKind::R2CPost: e = launch_r2c_post(s.real, src, dst, stream); break;
             case StepKind::C2RPre: e = launch_c2r_pre(s.real, src, dst, stream); break;
-            case StepKind::ChirpPre: e = launch_chirp_pre(s.chirp, src, dst, stream); break;
-            case StepKind::SpecMul: e = launch_spectrum_mul(s.chirp, dst, stream); break;
-            case StepKind::ChirpPost: e = launch_chirp_post(s.chirp, src, dst, stream); break;
+            case StepKind::ChirpLine: e = launch_chirp_line(s.chirp, src, dst, stream); break;
+            case StepKind::ChirpColsIn: e = launch_chirp_cols_in(s.chirp, src, dst, stream); break;
+            case StepKind::ChirpRows: e = launch_chirp_rows(s.chirp, dst, stream); break;
+            case StepKind::ChirpColsOut: e = launch_chirp_cols_out(s.chirp, src, dst, stream); break;
             case StepKind::Scale: e = launch_scale(dst, s.count, s.scale, stream); break;
             case StepKind::Chain:
             {

@@ -1,5 +1,5 @@
-// Elementwise passes around the line-FFT kernel: the real <-> half-length complex recombination of R2C/C2R and the
-// three chirp passes of Bluestein. All are streaming, HBM-bound grid-stride kernels.
+// Elementwise passes around the line-FFT kernel: the real <-> half-length complex recombination of R2C/C2R,
+// scaling and split-complex operands. All are streaming, HBM-bound grid-stride kernels.
 
 #include "codelets.cuh"
 #include "index.cuh"
@@ -111,64 +111,6 @@ __global__ void c2r_pre_kernel(const RealRecombine p, const float2* in, float2* 
     }
 }
 
-// a_k = x_k conj(chirp_k) (x conjugated first for the inverse), zero-padded to m (bluestein.hpp:95-106).
-__global__ void chirp_pre_kernel(const ChirpDesc p, const float2* x, float2* w)
-{
-    const long long total = p.m * p.batch;
-    const float2* ch = static_cast<const float2*>(p.chirp);
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x)
-    {
-        const long long t = idiv(i, p.m);
-        const long long k = i - t * p.m;
-        float2 r = make_float2(0.f, 0.f);
-        if (k < p.n)
-        {
-            float2 v = x[t * p.xdist + k];
-            if (p.conj)
-                v.y = -v.y;
-            const float2 c = ch[k];
-            r = make_float2(v.x * c.x + v.y * c.y, v.y * c.x - v.x * c.y);
-        }
-        w[t * p.wdist + k] = r;
-    }
-}
-
-// C = A * FFT_m(b) (bluestein.hpp:109-116).
-__global__ void spectrum_mul_kernel(const ChirpDesc p, float2* w)
-{
-    const long long total = p.m * p.batch;
-    const float2* bf = static_cast<const float2*>(p.bfft);
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x)
-    {
-        const long long t = idiv(i, p.m);
-        const long long k = i - t * p.m;
-        float2* wt = w + t * p.wdist;
-        wt[k] = cmul(wt[k], bf[k]);
-    }
-}
-
-// X_k = conj(chirp_k) c_k scale, conjugated for the inverse (bluestein.hpp:121-134).
-__global__ void chirp_post_kernel(const ChirpDesc p, const float2* w, float2* x)
-{
-    const long long total = p.n * p.batch;
-    const float2* ch = static_cast<const float2*>(p.chirp);
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x)
-    {
-        const long long t = idiv(i, p.n);
-        const long long k = i - t * p.n;
-        const float2 v = w[t * p.wdist + k];
-        const float2 c = ch[k];
-        float yr = (v.x * c.x + v.y * c.y) * p.scale;
-        float yi = (v.y * c.x - v.x * c.y) * p.scale;
-        if (p.conj)
-            yi = -yi;
-        x[t * p.xdist + k] = make_float2(yr, yi);
-    }
-}
-
 __global__ void scale_kernel(float2* data, long long count, float s)
 {
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < count;
@@ -191,26 +133,6 @@ cudaError_t launch_c2r_pre(const RealRecombine& p, const void* in, void* z, cuda
     const long long work = (p.h / 2 + 1) * p.batch;
     c2r_pre_kernel<<<grid_for(work, 256), 256, 0, stream>>>(p, static_cast<const float2*>(in),
                                                               static_cast<float2*>(z));
-    return cudaGetLastError();
-}
-
-cudaError_t launch_chirp_pre(const ChirpDesc& p, const void* x, void* w, cudaStream_t stream)
-{
-    chirp_pre_kernel<<<grid_for(p.m * p.batch, 256), 256, 0, stream>>>(p, static_cast<const float2*>(x),
-                                                                         static_cast<float2*>(w));
-    return cudaGetLastError();
-}
-
-cudaError_t launch_spectrum_mul(const ChirpDesc& p, void* w, cudaStream_t stream)
-{
-    spectrum_mul_kernel<<<grid_for(p.m * p.batch, 256), 256, 0, stream>>>(p, static_cast<float2*>(w));
-    return cudaGetLastError();
-}
-
-cudaError_t launch_chirp_post(const ChirpDesc& p, const void* w, void* x, cudaStream_t stream)
-{
-    chirp_post_kernel<<<grid_for(p.n * p.batch, 256), 256, 0, stream>>>(p, static_cast<const float2*>(w),
-                                                                          static_cast<float2*>(x));
     return cudaGetLastError();
 }
 

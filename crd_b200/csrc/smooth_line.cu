@@ -30,9 +30,6 @@ constexpr RadixCost kRadices[] = {{2, 2.0},   {3, 4.7},   {4, 4.0},   {5, 7.6}, 
                                   {16, 10.5}, {18, 14.0}, {20, 11.6}, {21, 14.1}, {24, 11.7}, {25, 19.0}};
 constexpr double kStageCost = 14.0;     // a point: shared-memory round trip, twiddle
 constexpr double kButterflyCost = 25.0; // a butterfly: its indices and addresses
-// The wide build's fewer resident warps (96 registers): 720 8.10.9 67.6 us a 256 MiB batch, 240 16.15 49.5 against
-// 12.20 59.2, but 3000 12.10.25 78.8 against 10.10.6.5 97.0, a stage more.
-constexpr double kWideCost = 1.12;
 
 struct Best
 {
@@ -70,7 +67,7 @@ bool smooth_wide(const int* radix, int nstages)
     return false;
 }
 
-bool smooth_radices(long long n, std::vector<int>& out, double* arith)
+bool smooth_radices(long long n, std::vector<int>& out, double* arith, double wide_cost)
 {
     out.clear();
     if (n < 1)
@@ -78,7 +75,7 @@ bool smooth_radices(long long n, std::vector<int>& out, double* arith)
     if (n == 1)
         out.push_back(1);
     std::map<long long, Best> narrow, wide;
-    const double cn = cheapest(n, 16, narrow), cw = kWideCost * cheapest(n, 25, wide);
+    const double cn = cheapest(n, 16, narrow), cw = wide_cost * cheapest(n, 25, wide);
     std::map<long long, Best>& memo = cw < cn ? wide : narrow;
     if (arith != nullptr)
         *arith = std::min(cn, cw);
@@ -201,13 +198,17 @@ bool smooth_tile(const PassDesc& d, int lpc, SmoothSched* s, smooth::Tile* t)
     return true;
 }
 
-// Threads of a tile: as many as the registers allow the CTAs that shared memory allows, 128 to 512 (1000-point lines
-// along: 128 threads 68.8 us, 320 71.5; eight interleaved, three CTAs an SM: 320 threads 89.1 us, 416 93.2, two CTAs).
-int smooth_line_threads(const PassDesc& d, int lpc)
+// Threads of a tile: as many as the registers allow the CTAs an SM holds, whether shared memory or the grid sets their
+// number, 128 to 512 and no more than the tile has butterflies for (1000-point lines along: 128 threads 68.8 us, 320
+// 71.5; eight interleaved, three CTAs an SM: 320 threads 89.1 us, 416 93.2, two CTAs).
+int smooth_threads(const SmoothSched& s, int lpc, int smem_bytes, int regs, long long grid)
 {
-    const int regs = smooth_wide(d.radix, d.nstages) ? 96 : d.ftw_M != 0 ? 72 : 64;
-    const int ctas = std::max(1, 227 * 1024 / (smooth_line_smem(d, lpc) + 1024));
-    return std::clamp(65536 / regs / ctas / 32 * 32, 128, 512);
+    const long long fill = (grid + 147) / 148; // CTAs an SM that the grid has
+    const int ctas = static_cast<int>(std::clamp(227LL * 1024 / (smem_bytes + 1024), 1LL, std::max(1LL, fill)));
+    int most = 0;
+    for (int i = 0; i < s.ns; ++i)
+        most = std::max(most, (lpc * s.st[i].N + 31) / 32 * 32);
+    return std::min(std::clamp(65536 / regs / ctas / 32 * 32, 128, 512), most);
 }
 
 // Lines a CTA: along the lines, tiles of about 2200 points (many CTAs an SM hide each other's phases: 1000-point lines
@@ -241,6 +242,7 @@ cudaError_t launch_smooth_line(const PassDesc& d, int lpc, const void* in, void*
         return cudaErrorInvalidConfiguration;
     const int epi = d.ftw_M != 0 ? 2 : (d.conj_in != 0 || d.conj_out != 0 || d.scale != 1.0f) ? 1 : 0;
     const bool wide = smooth_wide(d.radix, d.nstages);
+    const int regs = wide ? 96 : epi == 2 ? 72 : 64; // the kernels' __maxnreg__
     using Fn = void (*)(const PassDesc, const SmoothSched, const smooth::Tile, const float2*, float2*);
     const Fn fns[2][3] = {{smooth::smooth_line_kernel<0, false>, smooth::smooth_line_kernel<1, false>,
                            smooth::smooth_line_kernel<2, false>},
@@ -253,7 +255,7 @@ cudaError_t launch_smooth_line(const PassDesc& d, int lpc, const void* in, void*
         if (e != cudaSuccess)
             return e;
     }
-    fn<<<static_cast<unsigned>(groups), smooth_line_threads(d, lpc), smem, stream>>>(
+    fn<<<static_cast<unsigned>(groups), smooth_threads(s, lpc, smem, regs, groups), smem, stream>>>(
         d, s, smooth::tile_of(d, s, lpc), static_cast<const float2*>(in), static_cast<float2*>(out));
     return cudaGetLastError();
 }

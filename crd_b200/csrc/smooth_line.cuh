@@ -292,6 +292,119 @@ __device__ __forceinline__ void run_tile(const SmoothSched& s, float2* sm, int s
     }
 }
 
+// ---- convolution: transform, filter, transform back ------------------------------------------------------------------
+//
+// y = conj(DFT(conj(DFT(x) H))). After the forward stages the frequency digits sit at their places, k1 most
+// significant; a stage of the second transform takes digit k_i of place i back to the output digit j_i, last stage
+// first, so it reads and writes the places of the forward stage and ends in the order the input had:
+//     v = DFT_R(conj(..)), then v_j *= W_{L R}^{j k}  (the forward stage's twiddles, after the butterfly)
+// The last forward stage and the first one back share their places: one round trip, the filter applied in registers.
+
+// The last stage of two or more, the filter (io.filter on the frequencies b + r N), and its way back.
+template <int R, class IO>
+__device__ __forceinline__ void turn_stage(const SmoothSched& s, const Lanes& ln, float2* sm, int sl, int sp, int lpc,
+                                           int lines, const IO& io)
+{
+    const SmoothStage& t = s.st[s.ns - 1];
+    const int total = lpc * t.N;
+    const float2* tw = static_cast<const float2*>(s.tw) + t.tw;
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < total; idx += blockDim.x)
+    {
+        int l, b;
+        place(ln, idx, t, l, b);
+        if (l >= lines)
+            continue;
+        float2* p = sm + l * sl + last_place(s, b) * sp;
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            v[r] = p[r * sp];
+        twiddle<R>(v, tw, t.L, b);
+        Dft<R>::run(v);
+        io.template filter<R>(v, l, b, t.N);
+        Dft<R>::run(v);
+        twiddle<R>(v, tw, t.L, b);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            p[r * sp] = v[r];
+    }
+}
+
+template <int R>
+__device__ __forceinline__ void mid_back(const SmoothSched& s, int i, const Lanes& ln, float2* sm, int sl, int sp,
+                                         int lpc, int lines)
+{
+    const SmoothStage& t = s.st[i];
+    const int total = lpc * t.N;
+    const int step = t.ni * sp;
+    const float2* tw = static_cast<const float2*>(s.tw) + t.tw;
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < total; idx += blockDim.x)
+    {
+        int l, b, k;
+        place(ln, idx, t, l, b);
+        if (l >= lines)
+            continue;
+        float2* p = sm + l * sl + mid_place(s, i, b, k) * sp;
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            v[r] = p[r * step];
+        Dft<R>::run(v);
+        twiddle<R>(v, tw, t.L, k);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            p[r * step] = v[r];
+    }
+}
+
+template <int R, class IO>
+__device__ __forceinline__ void first_back(const SmoothSched& s, const Lanes& ln, const float2* sm, int sl, int sp,
+                                           int lpc, int lines, const IO& io)
+{
+    const SmoothStage& t = s.st[0];
+    const int total = lpc * t.N;
+    const int step = s.p1 * sp;
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < total; idx += blockDim.x)
+    {
+        int l, b;
+        place(ln, idx, t, l, b);
+        if (l >= lines)
+            continue;
+        const float2* p = sm + l * sl + b * sp;
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            v[r] = p[r * step];
+        Dft<R>::run(v);
+        io.template put<R>(v, l, b, t.N);
+    }
+}
+
+// A whole tile of a schedule of two or more stages, every thread of the CTA, threads along the lines.
+template <bool WIDE, class IO>
+__device__ __forceinline__ void run_conv_tile(const SmoothSched& s, float2* sm, int sl, int sp, int lpc, int lines,
+                                              const Lanes& ln, const IO& io)
+{
+    with_radix<WIDE>(s.st[0].R, [&]<int R>() { first_stage<R>(s, ln, sm, sl, sp, lpc, lines, io); });
+    for (int i = 1; i < s.ns - 1; ++i)
+    {
+        __syncthreads();
+        with_radix<WIDE>(s.st[i].R, [&]<int R>() { mid_stage<R>(s, i, ln, sm, sl, sp, lpc, lines); });
+    }
+    __syncthreads();
+    with_radix<WIDE>(s.st[s.ns - 1].R, [&]<int R>() { turn_stage<R>(s, ln, sm, sl, sp, lpc, lines, io); });
+    for (int i = s.ns - 2; i >= 1; --i)
+    {
+        __syncthreads();
+        with_radix<WIDE>(s.st[i].R, [&]<int R>() { mid_back<R>(s, i, ln, sm, sl, sp, lpc, lines); });
+    }
+    __syncthreads();
+    with_radix<WIDE>(s.st[0].R, [&]<int R>() { first_back<R>(s, ln, sm, sl, sp, lpc, lines, io); });
+}
+
 // ---- a line pass (pass_desc.hpp) as the tile's input and output ---------------------------------------------------
 
 // EPI: 0 plain, 1 conjugations and scale, 2 also the four-step twiddle.
