@@ -18,6 +18,7 @@
 #include "../../include/crdfft.h"
 #include "kernels.hpp"
 #include "pass_desc.hpp"
+#include "smooth_line.cuh"
 #include "smooth_plan.hpp"
 #include "tuner.hpp"
 #include "learned.hpp"
@@ -143,9 +144,7 @@ struct Step
 // With use32, the lengths where a radix-32 schedule measured faster as a unit-stride single pass take it (one
 // exchange through shared memory fewer): 1024 = 32 32 (66 -> 94 % of HBM), 8192 = 32 16 16. (512, 16384 and 32 were
 // slower with radix-32 stages, and so were the strided passes of the four-step.)
-// group25: pairs of 5s as radix-25 stages (off for the uneven kernel, whose inlined stages run out of registers with
-// a 25-point butterfly: 3.57 -> 3.72 ms for its 20,000-transform batch, where the line kernels gain 7-18 %).
-bool radices_for(long long n, std::vector<int>& out, bool use32 = false, bool group25 = true)
+bool radices_for(long long n, std::vector<int>& out, bool use32 = false)
 {
     out.clear();
     if (n < 1)
@@ -177,7 +176,7 @@ bool radices_for(long long n, std::vector<int>& out, bool use32 = false, bool gr
         return false;
     // pairs of 5s as radix-25 stages and pairs of 3s as radix-9 stages (one exchange through shared memory fewer
     // each), each before the odd one left over
-    if (group25 && std::getenv("CRDFFT_NO_RADIX25") == nullptr)
+    if (std::getenv("CRDFFT_NO_RADIX25") == nullptr)
     {
         std::vector<int> grouped;
         size_t i = 0;
@@ -2415,11 +2414,12 @@ crdfft_status build_real_conv(Plan& p, const ConvReq& req)
     return CRDFFT_OK;
 }
 
-// The split of a long uneven-batch transform: n = n1 * n2 with both halves at most `cap`, closest to square, n2
-// preferring a multiple of 16 (whole column tiles).
+// The split of a long uneven-batch transform: n = n1 * n2 with both halves at most `cap`, by the narrow schedules' cost,
+// whole 16-row tiles of the transposed store, and halves long enough to fill a tile with 16 lines.
 bool uneven_split(long long n, long long cap, long long* n1, long long* n2)
 {
     double best = 1e300;
+    std::vector<int> rad;
     for (long long d = 2; d * d <= n; ++d)
     {
         if (n % d != 0 || d > cap || n / d > cap || !is_smooth(d) || !is_smooth(n / d))
@@ -2427,11 +2427,11 @@ bool uneven_split(long long n, long long cap, long long* n1, long long* n2)
         for (int o = 0; o < 2; ++o)
         {
             const long long a = o ? d : n / d, b = o ? n / d : d;
-            // halves the kernel has as compile-time stages first, then whole 16-column tiles, then near square
-            const double stat = (uneven_static_ok(static_cast<int>(a)) ? 1.0 : 0.0) +
-                                (uneven_static_ok(static_cast<int>(b)) ? 1.0 : 0.0);
-            const double score = -3.0 * stat + (b % 16 != 0 ? 10.0 : 0.0) +
-                                 std::fabs(std::log(static_cast<double>(a) / b));
+            double ca = 0.0, cb = 0.0;
+            if (!smooth_radices(a, rad, &ca, 1e9) || !smooth_radices(b, rad, &cb, 1e9))
+                continue;
+            const double score = ca + cb + (b % 16 != 0 ? 8.0 : 0.0) + (a % 16 != 0 ? 8.0 : 0.0) +
+                                 12.0 * std::max(0.0, std::log2(static_cast<double>(std::max(a, b)) / 256.0));
             if (score < best)
             {
                 best = score;
@@ -2441,76 +2441,6 @@ bool uneven_split(long long n, long long cap, long long* n1, long long* n2)
         }
     }
     return best < 1e299;
-}
-
-// The uneven kernel's variant for items of line length n: its compile-time stages (1) or the run-time stages (0).
-// CRDFFT_UNEVEN_STATIC=0/1 forces it; otherwise wisdom, else in measure and learned mode a timed choice (an uneven
-// plan of that length alone, each variant executed cold) that is remembered, else the compile-time stages.
-thread_local int t_uneven_force = -1;
-std::atomic<int> g_uneven_force{-1}; // crdfft_debug_uneven_variant
-
-crdfft_status create_uneven(const int64_t* sizes, int64_t count, const int64_t* offsets, Plan** out);
-
-int uneven_variant(long long n)
-{
-    if (!uneven_static_ok(static_cast<int>(n)))
-        return 0;
-    if (t_uneven_force >= 0)
-        return t_uneven_force;
-    if (g_uneven_force.load() >= 0)
-        return g_uneven_force.load();
-    static const int env = [] {
-        const char* e = std::getenv("CRDFFT_UNEVEN_STATIC");
-        return e != nullptr ? (std::atoi(e) != 0 ? 1 : 0) : -1;
-    }();
-    if (env >= 0)
-        return env;
-    std::ostringstream k;
-    k << "D|uneven|n" << n;
-    const std::string key = k.str();
-    DecompEntry w;
-    if (decomp_lookup(key, &w))
-        return w.kind == 2 ? 1 : 0;
-    const int mode = planner_mode();
-    if (mode == kPlannerEstimate || t_arena != nullptr)
-        return 1;
-    const long long count = std::max(1LL, std::min(8192LL, (64LL << 20) / (8 * n)));
-    std::vector<int64_t> sz(static_cast<size_t>(count), n);
-    float ms[2] = {-1.0f, -1.0f};
-    for (int v = 0; v < 2; ++v)
-    {
-        t_uneven_force = v;
-        Plan* tp = nullptr;
-        const crdfft_status st = create_uneven(sz.data(), count, nullptr, &tp);
-        t_uneven_force = -1;
-        if (st != CRDFFT_OK)
-            continue;
-        void* in = nullptr;
-        void* outb = nullptr;
-        if (cudaMalloc(&in, static_cast<size_t>(count * n) * 8) == cudaSuccess &&
-            cudaMalloc(&outb, static_cast<size_t>(count * n) * 8) == cudaSuccess &&
-            cudaMemset(in, 0, static_cast<size_t>(count * n) * 8) == cudaSuccess)
-        {
-            auto go = [&](cudaStream_t s) {
-                return run(*tp, in, outb, CRDFFT_FORWARD, s, nullptr) == CRDFFT_OK ? cudaSuccess
-                                                                                     : cudaErrorLaunchFailure;
-            };
-            ms[v] = time_cold(go);
-        }
-        cudaGetLastError();
-        cudaFree(in);
-        cudaFree(outb);
-        destroy_plan(tp);
-    }
-    if (ms[0] < 0.0f && ms[1] < 0.0f)
-        return 1;
-    const int pick = (ms[1] > 0.0f && (ms[0] < 0.0f || ms[1] <= ms[0])) ? 1 : 0;
-    char buf[160];
-    std::snprintf(buf, sizeof(buf), "%s uneven-variant run-time=%.6f compile-time=%.6f pick=%d", key.c_str(),
-                  static_cast<double>(ms[0]), static_cast<double>(ms[1]), pick);
-    planner_log_append(buf);
-    decomp_store(key, DecompEntry{pick ? 2 : 1, 0, ms[pick]});
-    return pick;
 }
 
 template <typename T> crdfft_status upload_vec(Plan& p, const std::vector<T>& v, const T** out)
@@ -2527,17 +2457,15 @@ template <typename T> crdfft_status upload_vec(Plan& p, const std::vector<T>& v,
     return CRDFFT_OK;
 }
 
-// The uneven batch's work list (uneven.cu): transforms up to kUnevenSingle points grouped by length into CTA-sized
-// items; longer ones (7-smooth, up to kUnevenSingle^2) as four-step column and row tiles through a workspace region
-// of their own.
-// List order: every COL item (longest transforms first), then SMALL items (longest first), then ROW items.
+// The uneven batch's work list (uneven.cu): transforms up to kUnevenTile points grouped by length into CTA-sized
+// items; longer ones (7-smooth, both halves up to kUnevenTile) as four-step column and row tiles through a workspace
+// region of their own. List order: the long transforms' COL items (longest first), each transform's ROW items as soon
+// as more than the resident CTAs' items have followed its last COL item; the SMALL items (longest first) between the
+// last COL items and the ROW items still to come.
 crdfft_status build_uneven(Plan& p, const int64_t* sizes, int64_t count, const int64_t* offsets)
 {
-    p.use32 = false; // the uneven kernel's stages run 16 points a thread
-    const int threads = uneven_threads();
-    const long long kUnevenSingle = 16LL * threads; // the longest line one item transforms (16 points a thread)
     std::map<long long, int> sched_of;
-    std::vector<UnevenSched> scheds;
+    std::vector<SmoothSched> scheds;
     auto sched_index = [&](long long n, int* idx) -> crdfft_status {
         auto it = sched_of.find(n);
         if (it != sched_of.end())
@@ -2546,17 +2474,15 @@ crdfft_status build_uneven(Plan& p, const int64_t* sizes, int64_t count, const i
             return CRDFFT_OK;
         }
         std::vector<int> rad;
-        if (!radices_for(n, rad, false, false) || n > kUnevenSingle || static_cast<int>(rad.size()) > kMaxStages)
+        if (n > kUnevenTile || !smooth_radices(n, rad, nullptr, 1e9)) // the kernel holds the narrow radices
             return CRDFFT_UNSUPPORTED_SIZE;
-        UnevenSched sc{};
-        sc.n = static_cast<int>(n);
-        sc.variant = uneven_variant(n);
-        sc.nstages = static_cast<int>(rad.size());
-        for (size_t i = 0; i < rad.size(); ++i)
-            sc.radix[i] = rad[i];
-        const crdfft_status st = twiddle_table(p, rad, &sc.tw);
+        const void* tw = nullptr;
+        const crdfft_status st = twiddle_table(p, rad, &tw);
         if (st != CRDFFT_OK)
             return st;
+        SmoothSched sc{};
+        if (!smooth_sched(static_cast<int>(n), rad.data(), static_cast<int>(rad.size()), tw, &sc))
+            return CRDFFT_UNSUPPORTED_SIZE;
         *idx = static_cast<int>(scheds.size());
         sched_of[n] = *idx;
         scheds.push_back(sc);
@@ -2571,58 +2497,74 @@ crdfft_status build_uneven(Plan& p, const int64_t* sizes, int64_t count, const i
             return CRDFFT_UNSUPPORTED_SIZE;
         if (offsets[t] < 0)
             return CRDFFT_INVALID_ARG;
-        if (n <= kUnevenSingle)
+        if (n <= kUnevenTile)
             small[n].push_back(t);
         else
             large.push_back(t);
     }
     std::stable_sort(large.begin(), large.end(), [&](long long a, long long b) { return sizes[a] > sizes[b]; });
-    std::vector<UnevenItem> col, mid, row;
-    std::vector<long long> line_off;
-    std::vector<const void*> fh, fl;
-    std::map<long long, int> ftw_of;
+    int maxsmem = 1024;
+    // An item's tile of `lpc` lines of schedule s: across = the lanes run across the lines (a power of two of them).
+    auto set_tile = [&](UnevenItem& it, int s, int lpc, bool in_across, bool out_across) {
+        const SmoothSched& sc = scheds[static_cast<size_t>(s)];
+        const int places = sc.st[0].R * sc.p1;
+        int lg = 0;
+        while ((1 << (lg + 1)) <= lpc)
+            ++lg;
+        it.sched = s;
+        it.lpc = lpc;
+        it.sp = in_across ? lpc : 1;
+        it.sl = in_across ? 1 : places | 1;
+        it.first = in_across ? lg : -1;
+        it.last = out_across ? lg : -1;
+        maxsmem = std::max(maxsmem, lpc * (places | 1) * 8);
+    };
+    auto tile_lines = [](long long n) { // a power of two, up to 32 lines of a kUnevenTile tile
+        int l = 1;
+        while (l < 32 && 2 * l * n <= kUnevenTile)
+            l *= 2;
+        return l;
+    };
+    struct Split
+    {
+        long long n1, n2;
+        int s1, s2;
+        const void* hi;
+        const void* lo;
+    };
+    std::map<long long, Split> split_of;
+    std::vector<std::vector<UnevenItem>> cols(large.size()), rows(large.size());
     long long scratch = 0;
-    int maxsmem = 0;
     for (size_t li = 0; li < large.size(); ++li)
     {
         const long long t = large[li];
         const long long n = sizes[t];
-        long long n1 = 0, n2 = 0;
-        if (!uneven_split(n, kUnevenSingle, &n1, &n2))
-            return CRDFFT_UNSUPPORTED_SIZE;
-        int s1 = 0, s2 = 0;
-        crdfft_status st = sched_index(n1, &s1);
-        if (st == CRDFFT_OK)
-            st = sched_index(n2, &s2);
-        if (st != CRDFFT_OK)
-            return st;
-        int fidx;
-        auto fit = ftw_of.find(n);
-        if (fit == ftw_of.end())
+        auto found = split_of.find(n);
+        if (found == split_of.end())
         {
-            const void* hi = nullptr;
-            const void* lo = nullptr;
-            st = four_step_tables(p, n, n1, n2, &hi, &lo);
+            Split sp{};
+            if (!uneven_split(n, kUnevenTile, &sp.n1, &sp.n2))
+                return CRDFFT_UNSUPPORTED_SIZE;
+            crdfft_status st = sched_index(sp.n1, &sp.s1);
+            if (st == CRDFFT_OK)
+                st = sched_index(sp.n2, &sp.s2);
+            if (st == CRDFFT_OK)
+                st = four_step_tables(p, n, sp.n1, sp.n2, &sp.hi, &sp.lo);
             if (st != CRDFFT_OK)
                 return st;
-            fidx = static_cast<int>(fh.size());
-            fh.push_back(hi);
-            fl.push_back(lo);
-            ftw_of[n] = fidx;
+            found = split_of.emplace(n, sp).first;
         }
-        else
-            fidx = fit->second;
+        const Split& sp = found->second;
+        const long long n1 = sp.n1, n2 = sp.n2;
         const long long base = offsets[t];
         const long long reg = scratch;
-        scratch += (n + 1) / 2 * 2;
-        const int lc = std::max(1, std::min(threads / static_cast<int>((n1 + 15) / 16),
-                                            kMaxSmemBytes / (pass_line_pitch(static_cast<int>(n1)) * 8)));
-        int ncol = 0;
-        for (long long q0 = 0; q0 < n2; q0 += lc, ++ncol)
+        scratch += (n + 15) / 16 * 16; // each region on its own 128-byte lines
+        const int lc = tile_lines(n1), lr = tile_lines(n2);
+        for (long long q0 = 0; q0 < n2; q0 += lc)
         {
             UnevenItem it{};
             it.kind = kUnevenCol;
-            it.sched = s1;
+            set_tile(it, sp.s1, lc, true, true);
             it.lines = static_cast<int>(std::min<long long>(lc, n2 - q0));
             it.line_table = -1;
             it.in_base = base + q0;
@@ -2633,17 +2575,15 @@ crdfft_status build_uneven(Plan& p, const int64_t* sizes, int64_t count, const i
             it.out_estride = n2;
             it.transform = static_cast<int>(li);
             it.q0 = static_cast<int>(q0);
-            it.ftw = fidx;
-            col.push_back(it);
-            maxsmem = std::max(maxsmem, it.lines * pass_line_pitch(static_cast<int>(n1)) * 8);
+            it.ftw_hi = sp.hi;
+            it.ftw_lo = sp.lo;
+            cols[li].push_back(it);
         }
-        const int lr = std::max(1, std::min(threads / static_cast<int>((n2 + 15) / 16),
-                                            kMaxSmemBytes / (pass_line_pitch(static_cast<int>(n2)) * 8)));
         for (long long k0 = 0; k0 < n1; k0 += lr)
         {
             UnevenItem it{};
             it.kind = kUnevenRow;
-            it.sched = s2;
+            set_tile(it, sp.s2, lr, false, true);
             it.lines = static_cast<int>(std::min<long long>(lr, n1 - k0));
             it.line_table = -1;
             it.in_base = reg + k0 * n2;
@@ -2653,12 +2593,13 @@ crdfft_status build_uneven(Plan& p, const int64_t* sizes, int64_t count, const i
             it.out_ldist = 1;
             it.out_estride = n1;
             it.transform = static_cast<int>(li);
-            it.need = ncol + (g_debug_stall.load() ? 1 : 0); // the test hook asks for a COL item that never comes
-            it.ftw = -1;
-            row.push_back(it);
-            maxsmem = std::max(maxsmem, it.lines * pass_line_pitch(static_cast<int>(n2)) * 8);
+            // (the test hook asks for a COL item that never comes)
+            it.need = static_cast<int>(cols[li].size()) + (g_debug_stall.load() ? 1 : 0);
+            rows[li].push_back(it);
         }
     }
+    std::vector<UnevenItem> mid;
+    std::vector<long long> line_off;
     for (auto& kv : small)
     {
         const long long n = kv.first;
@@ -2666,57 +2607,62 @@ crdfft_status build_uneven(Plan& p, const int64_t* sizes, int64_t count, const i
         const crdfft_status st = sched_index(n, &sidx);
         if (st != CRDFFT_OK)
             return st;
-        const int lpi = std::max(1, std::min(threads / static_cast<int>((n + 15) / 16),
-                                             kMaxSmemBytes / (pass_line_pitch(static_cast<int>(n)) * 8)));
+        const int lpi = static_cast<int>(std::clamp<long long>(kUnevenTile / n, 1, kUnevenLines));
         const std::vector<long long>& ts = kv.second;
-        for (size_t i = 0; i < ts.size(); i += lpi)
+        for (size_t i = 0; i < ts.size(); i += static_cast<size_t>(lpi))
         {
             UnevenItem it{};
             it.kind = kUnevenSmall;
-            it.sched = sidx;
-            it.lines = static_cast<int>(std::min<size_t>(lpi, ts.size() - i));
+            set_tile(it, sidx, lpi, false, false);
+            it.lines = static_cast<int>(std::min<size_t>(static_cast<size_t>(lpi), ts.size() - i));
             it.line_table = static_cast<int>(line_off.size());
             for (int a = 0; a < it.lines; ++a)
-                line_off.push_back(offsets[ts[i + a]]);
+                line_off.push_back(offsets[ts[i + static_cast<size_t>(a)]]);
             it.in_estride = 1;
             it.out_estride = 1;
             it.transform = -1;
-            it.ftw = -1;
             mid.push_back(it);
-            maxsmem = std::max(maxsmem, it.lines * pass_line_pitch(static_cast<int>(n)) * 8);
         }
     }
+    p.usmem = maxsmem;
+    const long long resident = uneven_resident(maxsmem);
+    if (resident < 1)
+        return CRDFFT_LAUNCH;
     std::vector<UnevenItem> items;
-    items.insert(items.end(), col.begin(), col.end());
+    std::vector<size_t> last_col(large.size(), 0);
+    size_t next_row = 0;
+    for (size_t li = 0; li < large.size(); ++li)
+    {
+        items.insert(items.end(), cols[li].begin(), cols[li].end());
+        last_col[li] = items.size();
+        while (next_row < li && items.size() > last_col[next_row] + static_cast<size_t>(resident))
+        {
+            items.insert(items.end(), rows[next_row].begin(), rows[next_row].end());
+            ++next_row;
+        }
+    }
     items.insert(items.end(), mid.begin(), mid.end());
-    items.insert(items.end(), row.begin(), row.end());
+    for (; next_row < large.size(); ++next_row)
+        items.insert(items.end(), rows[next_row].begin(), rows[next_row].end());
     UnevenDesc& u = p.udesc;
     crdfft_status st = upload_vec(p, items, &u.items);
     if (st == CRDFFT_OK)
         st = upload_vec(p, scheds, &u.scheds);
     if (st == CRDFFT_OK)
         st = upload_vec(p, line_off, &u.line_off);
-    if (st == CRDFFT_OK)
-        st = upload_vec(p, fh, &u.tables.ftw_hi);
-    if (st == CRDFFT_OK)
-        st = upload_vec(p, fl, &u.tables.ftw_lo);
-    std::vector<int> counters(1 + large.size(), 0);
+    std::vector<int> counters(std::max<size_t>(1, large.size()), 0);
     const int* cdev = nullptr;
     if (st == CRDFFT_OK)
         st = upload_vec(p, counters, &cdev);
     if (st != CRDFFT_OK)
         return st;
-    u.counter = const_cast<int*>(cdev);
-    u.done = u.counter + 1;
+    u.done = const_cast<int*>(cdev);
     u.err = p.err;
     u.nitems = static_cast<int>(items.size());
     u.ntransforms = static_cast<int>(large.size());
     u.spin_limit = g_debug_stall.load() ? (1 << 10) : (1 << 24);
     u.conj = 0;
     u.scale = 1.0f;
-    // two item slots (one transformed while the next one's loads land) and the run-time stages' second buffer
-    u.slot_elems = (std::max(maxsmem, 1024) + 127) / 128 * 128 / 8;
-    p.usmem = 3 * u.slot_elems * 8;
     p.ws_bytes = static_cast<size_t>(scratch) * 8;
     p.uneven = true;
     p.algorithm = "uneven-batch";
@@ -2727,7 +2673,7 @@ crdfft_status build_uneven(Plan& p, const int64_t* sizes, int64_t count, const i
     return CRDFFT_OK;
 }
 
-// The uneven-batch plan (crdfft_plan_create_uneven); also the timing plans of uneven_variant.
+// The uneven-batch plan (crdfft_plan_create_uneven).
 crdfft_status create_uneven(const int64_t* sizes, int64_t count, const int64_t* offsets, Plan** out)
 {
     *out = nullptr;
@@ -3722,7 +3668,7 @@ void crdfft_debug_stall_waits(int32_t on) { g_debug_stall.store(on ? 1 : 0); }
 
 void crdfft_set_planner_mode(int32_t mode) { set_planner_mode(mode); }
 
-void crdfft_debug_uneven_variant(int32_t variant) { g_uneven_force.store(variant < 0 ? -1 : (variant ? 1 : 0)); }
+void crdfft_debug_uneven_variant(int32_t) {} // one form of stages: nothing to choose
 
 crdfft_status crdfft_set_decomposition(int64_t n, int32_t kind, int64_t n1)
 {

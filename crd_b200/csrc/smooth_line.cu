@@ -69,32 +69,52 @@ bool smooth_wide(const int* radix, int nstages)
 
 bool smooth_radices(long long n, std::vector<int>& out, double* arith, double wide_cost)
 {
+    struct Schedule
+    {
+        std::vector<int> radices;
+        double cost = 0.0;
+    };
+    thread_local std::map<std::pair<long long, double>, Schedule> memo; // a few hundred line lengths
     out.clear();
     if (n < 1)
         return false;
-    if (n == 1)
-        out.push_back(1);
-    std::map<long long, Best> narrow, wide;
-    const double cn = cheapest(n, 16, narrow), cw = wide_cost * cheapest(n, 25, wide);
-    std::map<long long, Best>& memo = cw < cn ? wide : narrow;
-    if (arith != nullptr)
-        *arith = std::min(cn, cw);
-    for (long long m = n; m > 1;)
+    auto it = memo.find({n, wide_cost});
+    if (it == memo.end())
     {
-        const Best& b = memo[m];
-        if (b.R == 0)
-            return false;
-        out.push_back(b.R);
-        m /= b.R;
+        Schedule s;
+        std::map<long long, Best> narrow, wide;
+        const double cn = cheapest(n, 16, narrow), cw = wide_cost * cheapest(n, 25, wide);
+        std::map<long long, Best>& pick = cw < cn ? wide : narrow;
+        s.cost = std::min(cn, cw);
+        if (n == 1)
+            s.radices.push_back(1);
+        for (long long m = n; m > 1;)
+        {
+            const Best& b = pick[m];
+            if (b.R == 0)
+                return false;
+            s.radices.push_back(b.R);
+            m /= b.R;
+        }
+        // Largest first (most loads in flight a thread, and the last stage's runs n / Rs in global memory are long),
+        // the smallest in the middle: 60 as 12.5 51.6 us against 4.15 62.6, 5000 as 25.10.20 83.2 against 10.20.25
+        // 89.1.
+        std::sort(s.radices.rbegin(), s.radices.rend());
+        if (s.radices.size() > 2)
+            std::swap(s.radices[1], s.radices.back());
+        if (n > 65535)
+        {
+            out = s.radices;
+            if (arith != nullptr)
+                *arith = s.cost;
+            return out.size() <= static_cast<size_t>(kSmoothStages);
+        }
+        it = memo.emplace(std::make_pair(n, wide_cost), s).first;
     }
-    if (out.size() > static_cast<size_t>(kSmoothStages))
-        return false;
-    // Largest first (most loads in flight a thread, and the last stage's runs n / Rs in global memory are long), the
-    // smallest in the middle: 60 as 12.5 51.6 us against 4.15 62.6, 5000 as 25.10.20 83.2 against 10.20.25 89.1.
-    std::sort(out.rbegin(), out.rend());
-    if (out.size() > 2)
-        std::swap(out[1], out.back());
-    return true;
+    out = it->second.radices;
+    if (arith != nullptr)
+        *arith = it->second.cost;
+    return out.size() <= static_cast<size_t>(kSmoothStages);
 }
 
 bool smooth_sched(int n, const int* radix, int nstages, const void* tw, SmoothSched* out)

@@ -444,8 +444,8 @@ crdfft_status crdfft_self_check(void);
 void crdfft_debug_self_check_mismatch(int32_t on);
 void crdfft_debug_self_check_reset(void);
 
-/* Test hook: uneven-batch plans created from now on run their power-of-two line lengths on the run-time stages (0)
- * or on the compile-time stages (1); -1 returns the choice to the planner. */
+/* Test hook of a choice the uneven-batch plans once had (run-time or compile-time stages); they have one form, so any
+ * value is accepted and changes nothing. */
 void crdfft_debug_uneven_variant(int32_t variant);
 
 /* Test hook: make the k-th device allocation from now fail (k >= 1), as if the device were out of memory; 0 turns

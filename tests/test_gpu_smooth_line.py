@@ -90,3 +90,25 @@ def test_four_step(dev, n, n1):
     for inverse in (False, True):
         got = run(x, plan, cf.INVERSE if inverse else cf.FORWARD)
         assert oracle.rel_l2(got, want(x, inverse)) <= 1e-6
+
+
+@pytest.mark.parametrize("sizes", [(2,), (4096, 2, 3, 4200), (4116, 16, 16, 16384), (65536,) * 3 + (27,) * 200,
+                                   (4900, 8192 * 7, 343 * 343, 3 ** 9, 5 ** 6)])
+def test_uneven_items(dev, sizes):
+    """The uneven batch's tiles (crd_b200/csrc/uneven.cu): one item only, the longest single line and the next length, lines
+    that leave a tile partly empty, halves with 3 and 4 stages, a transform whose own CTA takes its columns and rows."""
+    import torch
+
+    import crd_b200 as cf
+
+    plan = cf.UnevenPlan(list(sizes))
+    x = oracle.lcg_complex64(sum(sizes), plan.total)
+    t = torch.from_numpy(x).cuda()
+    for inverse in (False, True):
+        out = torch.zeros_like(t)
+        for _ in range(2):
+            plan.execute(t, out, cf.INVERSE if inverse else cf.FORWARD)
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        for n, at in list(zip(plan.sizes, plan.offsets))[:8]:
+            assert oracle.rel_l2(got[at:at + n], oracle.fft64(x[at:at + n], inverse)) <= 1e-6, n
