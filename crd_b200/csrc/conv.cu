@@ -13,6 +13,7 @@
 #include "dyn_stage.cuh"
 #include "kernels.hpp"
 #include "line_fft.cuh"
+#include "real_pair.cuh"
 
 namespace crdfft
 {
@@ -210,6 +211,89 @@ __global__ void __launch_bounds__(kMaxThreads)
     }
 }
 
+// The same for a real wavelet: X and K are spectra of real sequences, so w is real and its FFT of n = 2M points is an
+// M-point one (real_pair.cuh): Y = X K at k and M - k, k <= M/2, gives the pairs Q, and conj(FFT(conj Q)) holds
+// w[2m] + i w[2m + 1]. Half the arithmetic and half the shared memory of the complex form, whose 8192-point lines left
+// one 128-register CTA of 256 threads doing one line's stages at a time (64 x 64 lines: 180 -> 115 us a pass); the
+// coefficients' imaginary parts are the exact 0 they stand for.
+template <class S, int P>
+__global__ void __launch_bounds__(256, P == 16 ? 4 : 2)
+    cwt_real_line_kernel(const PassDesc d, const float2* __restrict__ X, const float2* __restrict__ K,
+                         const float2* __restrict__ wn, const CwtScale* __restrict__ scales, long long nscales,
+                         long long nsamples, float inv_n, float2* __restrict__ gout)
+{
+    extern __shared__ float2 sm[];
+    constexpr int M = S::n;
+    constexpr int T = M / P;
+    const int lpc = blockDim.x / T;
+    const int tid = threadIdx.x;
+    const int ll = tid / T;
+    const int jt = tid - ll * T;
+    const long long line = static_cast<long long>(blockIdx.x) * lpc + ll;
+    Ctx c;
+    c.ok = line < d.lines;
+    c.q = 0;
+    c.in = X;
+    c.out = gout;
+    c.jt = jt;
+    c.T = T;
+    init_scales(d, c);
+    const LayRow<1> lay{sm + ll * line_pitch(M)};
+    const long long sig = idiv(line, nscales), s = line - sig * nscales;
+    if (c.ok)
+    {
+        const float2* x = X + sig * (2 * M);
+        const float2* h = K + s * (2 * M);
+        auto y = [&](int k) { return cmul(__ldg(x + k), __ldg(h + k)); };
+#pragma unroll 4
+        for (int k = jt; k <= M / 2; k += T)
+        {
+            const float2 w = k == 0 ? make_float2(1.0f, 0.0f) : __ldg(wn + k);
+            float2 a, b;
+            c2r_pair(y(k), y(M - k), w, a, b);
+            lay.at(k) = conjf2(a);
+            if (k != 0 && M - k != k)
+                lay.at(M - k) = conjf2(b);
+        }
+    }
+    __syncthreads();
+    SchedRun<S>::template go<P, false, false, false, Kind<PassMap::Row, false>>(d, c, lay, M);
+    if (c.ok)
+    {
+        const CwtScale p = scales[s];
+        float2* o = gout + line * nsamples;
+        auto w = [&](int t) {
+            const float2* e = &lay.at(t >> 1);
+            return (t & 1) ? -e->y : e->x;
+        };
+        const float g = p.taps_ok ? p.amp * inv_n : 0.0f;
+        const int off = p.taps_ok ? static_cast<int>(p.off) : 0;
+        for (int i = jt; i < static_cast<int>(nsamples); i += T)
+            __stcs(o + i, make_float2(p.taps_ok ? g * (w(off + i + 1) - w(off + i)) : 0.0f, 0.0f));
+    }
+}
+
+using CwtRealFn = void (*)(const PassDesc, const float2*, const float2*, const float2*, const CwtScale*, long long,
+                           long long, float, float2*);
+
+// The half-length schedules: 512 .. 8192-point transforms (longer ones run in rounds, cwt_plan.cpp).
+CwtRealFn cwt_real_select(const PassDesc& d, int* P)
+{
+    *P = 32;
+    if (same_radices(d, {32, 32}))
+        return cwt_real_line_kernel<Sched<32, 32>, 32>;
+    *P = 16;
+    if (same_radices(d, {16, 16}))
+        return cwt_real_line_kernel<Sched<16, 16>, 16>;
+    if (same_radices(d, {16, 8, 4}))
+        return cwt_real_line_kernel<Sched<16, 8, 4>, 16>;
+    if (same_radices(d, {16, 16, 8}))
+        return cwt_real_line_kernel<Sched<16, 16, 8>, 16>;
+    if (same_radices(d, {16, 16, 16}))
+        return cwt_real_line_kernel<Sched<16, 16, 16>, 16>;
+    return nullptr;
+}
+
 using CwtFn = void (*)(const PassDesc, const float2*, const float2*, const CwtScale*, long long, long long, float,
                        float2*);
 
@@ -357,6 +441,40 @@ cudaError_t launch_cwt_lines(const PassDesc& d, const void* X, const void* K, co
     fn<<<static_cast<unsigned>(groups), T * lpc, smem, stream>>>(
         d, static_cast<const float2*>(X), static_cast<const float2*>(K), scales, nscales, n,
         static_cast<float>(1.0 / static_cast<double>(d.n)), static_cast<float2*>(out));
+    return cudaGetLastError();
+}
+
+bool cwt_real_lines_supported(const PassDesc& d)
+{
+    int P = 0;
+    return lfft::cwt_real_select(d, &P) != nullptr;
+}
+
+cudaError_t launch_cwt_real_lines(const PassDesc& d, const void* X, const void* K, const void* wn,
+                                  const CwtScale* scales, long long nscales, long long n, void* out,
+                                  cudaStream_t stream)
+{
+    int P = 0;
+    lfft::CwtRealFn fn = lfft::cwt_real_select(d, &P);
+    if (fn == nullptr || n < 1 || n >= 2LL * d.n)
+        return cudaErrorInvalidConfiguration;
+    const int T = d.n / P;
+    const int lpc = 256 / T;
+    const int smem = lpc * lfft::line_pitch(d.n) * 8;
+    const long long groups = (d.lines + lpc - 1) / lpc;
+    if (groups <= 0)
+        return cudaSuccess;
+    if (groups > 0x7fffffffLL)
+        return cudaErrorInvalidConfiguration;
+    if (smem > 48 * 1024)
+    {
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess)
+            return e;
+    }
+    fn<<<static_cast<unsigned>(groups), T * lpc, smem, stream>>>(
+        d, static_cast<const float2*>(X), static_cast<const float2*>(K), static_cast<const float2*>(wn), scales, nscales,
+        n, static_cast<float>(0.5 / static_cast<double>(d.n)), static_cast<float2*>(out));
     return cudaGetLastError();
 }
 

@@ -33,6 +33,8 @@ struct crdfft_cwt_plan
     long long n = 0, count = 0, nscales = 0, lfft = 0;
     long long chunk = 0;                 // signals a product / inverse FFT / epilogue round takes
     bool fused = false;                  // one line kernel over all (signal, scale) lines (conv.cu)
+    bool real_lines = false;             // fused, real wavelet: half-length lines
+    void* roots = nullptr;               // real_lines: W_lfft^k, k <= lfft / 4
     crdfft_plan* lines_plan = nullptr;   // fused: the convolution plan whose line pass (stages, twiddles) it runs
     crdfft::PassDesc pass{};             // fused: that line pass, lines = count x nscales
     crdfft_plan* forward = nullptr;      // the signals' FFTs (batch count, in place on X)
@@ -48,7 +50,7 @@ struct crdfft_cwt_plan
         for (crdfft_plan* p : {forward, inverse, inverse_tail, lines_plan})
             if (p != nullptr)
                 crdfft_plan_destroy(p);
-        for (void* b : {spectra, X, W, static_cast<void*>(scales)})
+        for (void* b : {spectra, X, W, roots, static_cast<void*>(scales)})
             if (b != nullptr)
                 cudaFree(b);
     }
@@ -423,7 +425,39 @@ crdfft_status build(const crdfft_cwt_desc* d, const Geometry& g, crdfft_cwt_plan
     // the fused line kernel where the FFT length has a compile-time schedule: one launch, no filtered-sequence scratch
     const long long line_bytes = lfft * 8;
     crdfft_desc ld = line_desc(lfft, d->count * ns);
-    if (crdfft_conv_plan_create(&ld, 0, 1.0, &p->lines_plan) == CRDFFT_OK)
+    // (a real wavelet: the half-length line, its roots W_lfft^k beside it)
+    if (!g.w.complex_valued && lfft >= 4)
+    {
+        crdfft_desc hd = line_desc(lfft / 2, d->count * ns);
+        if (crdfft_conv_plan_create(&hd, 0, 1.0, &p->lines_plan) == CRDFFT_OK)
+        {
+            p->real_lines = crdfft::conv_line_pass(p->lines_plan, &p->pass) && crdfft::cwt_real_lines_supported(p->pass);
+            p->fused = p->real_lines;
+            if (!p->real_lines)
+            {
+                crdfft_plan_destroy(p->lines_plan);
+                p->lines_plan = nullptr;
+            }
+        }
+    }
+    if (p->real_lines)
+    {
+        std::vector<float> wn(static_cast<size_t>(lfft / 4 + 1) * 2);
+        for (long long k = 0; k <= lfft / 4; ++k)
+        {
+            const double a = -2.0 * M_PI * static_cast<double>(k) / static_cast<double>(lfft);
+            wn[static_cast<size_t>(2 * k)] = static_cast<float>(std::cos(a));
+            wn[static_cast<size_t>(2 * k + 1)] = static_cast<float>(std::sin(a));
+        }
+        if (cudaMalloc(&p->roots, wn.size() * 4) != cudaSuccess)
+        {
+            cudaGetLastError();
+            return CRDFFT_OOM;
+        }
+        if (cudaMemcpy(p->roots, wn.data(), wn.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess)
+            return CRDFFT_LAUNCH;
+    }
+    else if (crdfft_conv_plan_create(&ld, 0, 1.0, &p->lines_plan) == CRDFFT_OK)
     {
         p->fused = crdfft::conv_line_pass(p->lines_plan, &p->pass) && crdfft::cwt_lines_supported(p->pass);
         if (!p->fused)
@@ -536,6 +570,11 @@ crdfft_status crdfft_cwt_execute(crdfft_cwt_plan* plan, const float* x, void* co
     crdfft_status st = crdfft_execute(p.forward, p.X, p.X, CRDFFT_FORWARD, stream);
     if (st != CRDFFT_OK)
         return st;
+    if (p.real_lines)
+        return crdfft::launch_cwt_real_lines(p.pass, p.X, p.spectra, p.roots, p.scales, p.nscales, p.n, coeffs, s) ==
+                       cudaSuccess
+                   ? CRDFFT_OK
+                   : CRDFFT_LAUNCH;
     if (p.fused)
         return crdfft::launch_cwt_lines(p.pass, p.X, p.spectra, p.scales, p.nscales, p.n, coeffs, s) == cudaSuccess
                    ? CRDFFT_OK

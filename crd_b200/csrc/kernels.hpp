@@ -195,6 +195,12 @@ cudaError_t launch_cwt_diff(const void* W, const CwtScale* scales, void* out, lo
 // d.lines = signals x nscales lines of this launch. cwt_lines_supported: a compile-time schedule exists for d.
 bool conv_line_pass(crdfft_plan* plan, PassDesc* out);
 bool cwt_lines_supported(const PassDesc& d);
+// For a real wavelet (X and K then spectra of real sequences, 2 d.n values a line): d is the half-length line, wn holds
+// W_{2 d.n}^k for k <= d.n / 2.
+bool cwt_real_lines_supported(const PassDesc& d);
+cudaError_t launch_cwt_real_lines(const PassDesc& d, const void* X, const void* K, const void* wn,
+                                  const CwtScale* scales, long long nscales, long long n, void* out,
+                                  cudaStream_t stream);
 cudaError_t launch_cwt_lines(const PassDesc& d, const void* X, const void* K, const CwtScale* scales, long long nscales,
                              long long n, void* out, cudaStream_t stream);
 
