@@ -84,7 +84,13 @@ struct SpectralDesc
     float scale;        // 1 / (fs sum w^2)
     const float* win;   // nperseg window values
     const void* wn;     // float2 W_nperseg^k, k = 0 .. M/2 at least
+    int ppc;            // segment pairs a CTA (welch_pair.cu); 0: the segment-by-segment kernel
+    const void* pair_tw; // its stage twiddles
 };
+// Welch with two segments a complex transform (welch_pair.cu): false when the segment length has no kernel. ntiles: rows
+// of sums a signal, for launch_welch_finish.
+bool welch_pair_shape(int nperseg, long long count, long long nseg, std::vector<int>* radices, int* ntiles, int* ppc);
+cudaError_t launch_welch_pair(const SpectralDesc& sd, const void* x, void* part, cudaStream_t stream);
 bool spectral_shape(const PassDesc& d, int* P, int* lpc, int* threads, int* smem);
 cudaError_t launch_spectral(const PassDesc& d, const SpectralDesc& sd, int threads, int smem, const void* x,
                             void* out, cudaStream_t stream);

@@ -2857,6 +2857,13 @@ crdfft_status build_spectral(Plan& p, const crdfft_spectral_desc& s)
     sd.scale = static_cast<float>(1.0 / (s.fs * ss));
     sd.win = static_cast<const float*>(dwin);
     sd.wn = dwn;
+    std::vector<int> rad;
+    if (welch && welch_pair_shape(sd.nperseg, sd.count, sd.nseg, &rad, &sd.ntiles, &sd.ppc))
+    {
+        st = twiddle_table(p, rad, &sd.pair_tw);
+        if (st != CRDFFT_OK)
+            return st;
+    }
     sp.sdesc = sd;
     sp.sthreads = threads;
     sp.ssmem = smem;
@@ -3057,7 +3064,8 @@ crdfft_status run(Plan& p, const void* in, void* out, int dir, cudaStream_t stre
                 e = launch_conv(s.pass, s.shape.map, s.smap, src, spec, dst, stream);
                 break;
             case StepKind::Spectral:
-                e = launch_spectral(s.pass, s.sdesc, s.sthreads, s.ssmem, src, dst, stream);
+                e = s.sdesc.ppc > 0 ? launch_welch_pair(s.sdesc, src, dst, stream)
+                                    : launch_spectral(s.pass, s.sdesc, s.sthreads, s.ssmem, src, dst, stream);
                 break;
             case StepKind::WelchFinish: e = launch_welch_finish(s.sdesc, src, dst, stream); break;
             case StepKind::TmaCol: e = launch_tma_col(s.pass, src, dst, stream); break;

@@ -230,19 +230,36 @@ __global__ void __launch_bounds__(DYN ? kMaxThreads : kStaticThreads, DYN ? 1 : 
     }
 }
 
-// The per-CTA sums of each signal added in CTA order, divided by the segment count (spectral.hpp:158-171).
-__global__ void welch_finish_kernel(const float* __restrict__ part, float* __restrict__ psd, long long count,
-                                    int ntiles, int nfreq, float nseg)
+// The per-CTA sums of each signal added in a fixed order, divided by the segment count (spectral.hpp:158-171): eight
+// slices of consecutive rows, each in row order, then the slices in order (one thread over all the rows of a frequency
+// took 58 us for 16 signals x 1024 rows of 513).
+constexpr int kFinishFreqs = 32;
+constexpr int kFinishSlices = 8;
+__global__ void __launch_bounds__(kFinishFreqs* kFinishSlices)
+    welch_finish_kernel(const float* __restrict__ part, float* __restrict__ psd, long long count, int ntiles, int nfreq,
+                        float nseg)
 {
-    const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= count * nfreq)
-        return;
-    const long long g = idx / nfreq;
-    const int k = static_cast<int>(idx - g * nfreq);
-    const float* p = part + g * ntiles * static_cast<long long>(nfreq) + k;
+    __shared__ float sums[kFinishSlices][kFinishFreqs];
+    const long long idx = static_cast<long long>(blockIdx.x) * kFinishFreqs + threadIdx.x % kFinishFreqs;
+    const int slice = threadIdx.x / kFinishFreqs;
+    const bool ok = idx < count * nfreq;
     float acc = 0.0f;
-    for (int t = 0; t < ntiles; ++t)
-        acc += p[static_cast<long long>(t) * nfreq];
+    if (ok)
+    {
+        const long long g = idiv(idx, nfreq);
+        const int k = static_cast<int>(idx - g * nfreq);
+        const float* p = part + g * ntiles * static_cast<long long>(nfreq) + k;
+        const int each = (ntiles + kFinishSlices - 1) / kFinishSlices;
+        const int end = min(ntiles, (slice + 1) * each);
+        for (int t = slice * each; t < end; ++t)
+            acc += p[static_cast<long long>(t) * nfreq];
+    }
+    sums[slice][threadIdx.x % kFinishFreqs] = acc;
+    __syncthreads();
+    if (slice != 0 || !ok)
+        return;
+    for (int s = 1; s < kFinishSlices; ++s)
+        acc += sums[s][threadIdx.x];
     psd[idx] = acc / nseg;
 }
 
@@ -336,10 +353,10 @@ cudaError_t launch_welch_finish(const SpectralDesc& sd, const void* part, void* 
     const long long total = sd.count * nfreq;
     if (total <= 0)
         return cudaSuccess;
-    const long long blocks = (total + 255) / 256;
+    const long long blocks = (total + lfft::kFinishFreqs - 1) / lfft::kFinishFreqs;
     if (blocks > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    lfft::welch_finish_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
+    lfft::welch_finish_kernel<<<static_cast<unsigned>(blocks), lfft::kFinishFreqs * lfft::kFinishSlices, 0, stream>>>(
         static_cast<const float*>(part), static_cast<float*>(psd), sd.count, sd.ntiles, nfreq,
         static_cast<float>(sd.nseg));
     return cudaGetLastError();
