@@ -633,8 +633,15 @@ PassShape shape_with(long long n, int nstages, PassMap map, bool dl, bool ds, in
     sh.threads_per_line = T;
     // the compile-time-schedule kernel's pitch (at least the run-time kernel's, which sizes its own two buffers)
     auto tile_bytes = [&](int l) { return l * pass_cta_line_pitch(static_cast<int>(n), l) * 8; };
+    // The defaults, by timings of every candidate on 256 MiB (ms): rows stored along the lines in CTAs of 128 threads
+    // (1024 points 0.0892 against 0.1043 with 256, 512 0.088 / 0.098, 2048 0.092 / 0.102, 32 0.217 / 0.268); rows stored
+    // across the lines 256, whose runs in memory are twice as long; columns of up to 256 points, and of 1024 at 32 points
+    // a thread, 256 (256 points 0.096 / 0.133, 64 0.088 / 0.092), longer ones 512 threads, for runs of 32 bytes or more.
     if (lpc <= 0)
-        lpc = map == PassMap::Row ? std::max(1, 256 / T) : std::max(1, 512 / T);
+    {
+        const int threads = map == PassMap::Row ? (ds ? 128 : 256) : (n <= 256 || (P == 32 && n <= 1024)) ? 256 : 512;
+        lpc = std::max(1, threads / T);
+    }
     lpc = std::min(lpc, pass_lines_per_cta_limit());
     while (lpc > 1 && lpc * T > pass_threads_limit(P, n))
         --lpc;
@@ -726,7 +733,7 @@ bool heuristic_shape(const PassDesc& d, PassMap map, bool dl, bool ds, PassShape
         *out = smooth_shape(d, map, dl, ds);
         return true;
     }
-    const bool want32 = d.n > 8192 || (map == PassMap::Col && d.n >= 2048);
+    const bool want32 = d.n > 8192 || (map == PassMap::Col && d.n >= 1024); // (1024-point columns 0.156 ms, 0.182 at 16)
     if (want32)
     {
         const PassShape sh = shape_with(d.n, d.nstages, map, dl, ds, 32);
