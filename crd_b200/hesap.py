@@ -36,6 +36,8 @@ Inverse = INVERSE
 
 
 def _dir(direction) -> int:
+    if direction is FORWARD or direction is INVERSE:
+        return direction
     if isinstance(direction, str):
         direction = {"forward": FORWARD, "inverse": INVERSE}[direction.lower()]
     d = int(direction)
@@ -44,22 +46,31 @@ def _dir(direction) -> int:
     return d
 
 
-def _stream(stream) -> ctypes.c_void_p:
+# The raw handle of torch's current stream without building a torch.cuda.Stream around it, where this torch has the call:
+# a short transform's call is bound by the host (one 1024-point transform: 9.4 us a call through the Stream object and
+# ctypes pointer objects, of which the launch itself is about 3).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
+def _stream(stream) -> int:
     if stream is None:
+        if _raw_stream is not None and _raw_device is not None and torch.cuda.is_initialized():
+            return _raw_stream(_raw_device())
         stream = torch.cuda.current_stream()
     if isinstance(stream, torch.cuda.Stream):
-        return ctypes.c_void_p(stream.cuda_stream)
-    return ctypes.c_void_p(int(stream))
+        return stream.cuda_stream
+    return int(stream)
 
 
-def _ptr(t: torch.Tensor, dtype: torch.dtype, what: str) -> ctypes.c_void_p:
+def _ptr(t: torch.Tensor, dtype: torch.dtype, what: str) -> int:
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise ValueError(f"{what} must be a CUDA tensor")
     if t.dtype != dtype:
         raise ValueError(f"{what} must be {dtype}, got {t.dtype}")
     if not t.is_contiguous():
         raise ValueError(f"{what} must be contiguous")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 class _Handle:
