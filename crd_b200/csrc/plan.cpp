@@ -639,7 +639,7 @@ PassShape shape_with(long long n, int nstages, PassMap map, bool dl, bool ds, in
     // a thread, 256 (256 points 0.096 / 0.133, 64 0.088 / 0.092), longer ones 512 threads, for runs of 32 bytes or more.
     if (lpc <= 0)
     {
-        const int threads = map == PassMap::Row ? (ds ? 128 : 256) : (n <= 256 || (P == 32 && n <= 1024)) ? 256 : 512;
+        const int threads = map == PassMap::Row ? (ds || n <= 32 ? 128 : 256) : (n <= 256 || (P == 32 && n <= 1024)) ? 256 : 512;
         lpc = std::max(1, threads / T);
     }
     lpc = std::min(lpc, pass_lines_per_cta_limit());
@@ -1227,10 +1227,20 @@ crdfft_status make_pass_desc(Plan& p, long long n, long long lines, long long lp
     d.nstages = static_cast<int>(rad.size());
     for (size_t i = 0; i < rad.size(); ++i)
         d.radix[i] = rad[i];
-    if (line && !pass_has_static(d, 16) && !pass_has_static(d, 32))
+    const bool short_rows = line && n <= 32 && in.estride == 1 && out.estride == 1 && p.desc.precision == CRDFFT_PREC_FP32;
+    if (line && ((!pass_has_static(d, 16) && !pass_has_static(d, 32)) || short_rows))
     {
         if (!smooth_radices(n, rad) || static_cast<int>(rad.size()) > kMaxStages)
             return CRDFFT_UNSUPPORTED_SIZE;
+        // Rows of up to 32 points on both sides: two stages, whose threads share a row's 128-byte lines. As one radix a
+        // thread reads and writes a whole row by itself (256 MiB: 18 points 102 us, 24 117, 36 in two stages 58), and
+        // the compile-time 32-point kernel stages rows through shared memory both ways (111 us).
+        if (short_rows && n == 32)
+            rad = {4, 8};
+        else if (short_rows && rad.size() == 1)
+            for (int a = 2; a * a <= static_cast<int>(n); ++a)
+                if (n % a == 0)
+                    rad = {static_cast<int>(n) / a, a};
         d.nstages = static_cast<int>(rad.size());
         for (size_t i = 0; i < rad.size(); ++i)
             d.radix[i] = rad[i];

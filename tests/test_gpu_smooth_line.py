@@ -12,7 +12,7 @@ import oracle
 
 pytestmark = pytest.mark.gpu
 
-LENGTHS = (1, 3, 6, 7, 12, 14, 15, 18, 20, 21, 24, 25, 35, 49, 60, 100, 243, 343, 360, 625, 1000, 2401, 3125, 4200, 5000,
+LENGTHS = (1, 3, 6, 7, 12, 14, 15, 16, 18, 20, 21, 24, 25, 32, 35, 49, 60, 100, 243, 343, 360, 625, 1000, 2401, 3125, 4200, 5000,
            6144, 6561, 7203, 8000)
 
 
