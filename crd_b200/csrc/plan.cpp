@@ -291,7 +291,8 @@ bool column_split(long long n, long long* n1, long long* n2)
 // both halves within one CTA: the cheapest sum of two measured costs, us for 2^24 points above a common base. They are
 // a least-squares fit to every split of 33 lengths from 10^4 to 2^22 (924 timings); picking by them is 3.5 % off
 // the fastest split on average (17 % at worst), the closest-to-square rule it replaces 10 % (26 %): 107520 as
-// 105 x 1024 160.7 us, 210 x 512 141.4; 2^17 as 256 x 512 132.1, 128 x 1024 123.0.
+// 105 x 1024 160.7 us, 210 x 512 141.4; 2^17 as 256 x 512 132.1, 128 x 1024 123.0. (512 columns and 2048 rows stand
+// above their fit: 2^19 is 495.9 us for 2^26 points as 1024 x 512, 541.7 the other way round, 2^21 as 2048 x 1024.)
 // compiled: lengths with a compile-time schedule run it (the chirp convolution's passes never do).
 double split_pass_cost(long long n, bool rows, bool compiled);
 
@@ -304,7 +305,7 @@ double split_pass_cost_of(long long n, bool rows, bool compiled)
     };
     static const Static kStatic[] = {{16, -4.0, 0.1},   {32, 3.1, 26.0},     {64, 4.3, 1.4},      {105, 41.2, 34.9},
                                      {128, 10.4, 2.0},
-                                     {256, 21.2, -10.2}, {512, 35.9, -8.5},   {1024, 37.3, -13.8}, {2048, 81.4, 32.0},
+                                     {256, 21.2, -10.2}, {512, 45.0, -8.5},   {1024, 37.3, -13.8}, {2048, 81.4, 32.0},
                                      {4096, 99.2, 87.6}, {8192, 130.0, 130.0}, {16384, 250.0, 250.0}};
     for (const Static& s : kStatic)
         if (compiled && s.n == n)
