@@ -1397,8 +1397,8 @@ bool tma_col_enabled()
 }
 
 // L2 waves run round-robin over this many internal streams and workspace slots (CRDFFT_L2_LANES, 2 .. kMaxLanes).
-// Two measured best for 107520 (2.170 ms per 2 GiB; three lanes 2.286 with 24 MiB waves, 2.172 with 16 MiB, four
-// 2.422): more than about 48 MiB of waves in flight pushes the intermediates out of L2.
+// (2^26 points: three lanes of 24 MiB waves 516 us for 107520, 420 for 131072, two of 32 MiB 501 and 416; more than about
+// 96 MiB of waves in flight pushes the intermediates out of L2).
 int l2_lanes()
 {
     const char* e = std::getenv("CRDFFT_L2_LANES");
@@ -1424,7 +1424,11 @@ bool l2_waves()
     return on;
 }
 
-// The L2 wave size and the largest transform (bytes) that takes L2 waves; CRDFFT_L2_WAVE_BYTES and
+// Batches of more than this take L2 waves (two of them at least have to overlap).
+constexpr long long kL2WavesFrom = 48LL << 20;
+
+// The L2 wave size (two lanes, 2^26 points: 131072 416 us with 32 MiB waves, 428 with 24, 446 with 18; 107520 501 / 506 /
+// 522; 20160 439 / 455 / 490) and the largest transform (bytes) that takes L2 waves; CRDFFT_L2_WAVE_BYTES and
 // CRDFFT_L2_WAVE_MAX_TRANSFORM override them.
 long long env_bytes(const char* name, long long dflt)
 {
@@ -1439,7 +1443,7 @@ long long env_bytes(const char* name, long long dflt)
 }
 long long l2_wave_bytes()
 {
-    static const long long v = env_bytes("CRDFFT_L2_WAVE_BYTES", 24LL << 20);
+    static const long long v = env_bytes("CRDFFT_L2_WAVE_BYTES", 32LL << 20);
     return v;
 }
 long long l2_wave_max_transform()
@@ -1605,7 +1609,7 @@ crdfft_status plan_c2c_1d(Plan& p, long long n, long long batch, long long istri
     // one's pass 1 (and fills its tail). Otherwise one large wave at a time on the caller's stream.
     // (Transforms above 2 MiB are left to large waves: a 24 MiB wave of them is too few tiles to fill the GPU.)
     const bool l2w = l2_waves() && t_arena == nullptr && n * 8 <= l2_wave_max_transform() &&
-                     batch * n * 8 > 2 * l2_wave_bytes();
+                     batch * n * 8 > kL2WavesFrom;
     long long wave = std::max(1LL, (l2w ? l2_wave_bytes() : wave_bytes()) / (n * 8));
     wave = std::min(wave, batch);
     const int nl = l2_lanes();
