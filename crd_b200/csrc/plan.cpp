@@ -1611,7 +1611,9 @@ crdfft_status plan_c2c_1d(Plan& p, long long n, long long batch, long long istri
     const bool l2w = l2_waves() && t_arena == nullptr && n * 8 <= l2_wave_max_transform() &&
                      batch * n * 8 > kL2WavesFrom;
     long long wave = std::max(1LL, (l2w ? l2_wave_bytes() : wave_bytes()) / (n * 8));
-    wave = std::min(wave, batch);
+    // Waves of equal size: a short last one ran at a fraction of the rate (2^20 x 70, padded, as 64 and 6: 776 us).
+    const long long nwaves = (batch + wave - 1) / wave;
+    wave = (batch + nwaves - 1) / nwaves;
     const int nl = l2_lanes();
     *ws_need = (l2w ? nl : 1) * wave * n;
     int wi = 0;
