@@ -22,7 +22,8 @@
 // bounded anyway (spin_limit polls): one that runs out sets the plan's status word and skips the item.
 //
 // Two asynchronously filled 32 KB slots and out-of-place stages before: 215 instructions a point and pass, two CTAs an
-// SM, every intermediate through HBM. Now 95 instructions; bound by latency (33 % issue at 20 to 24 warps).
+// SM, every intermediate through HBM. Now 95 instructions; bound by latency (42 % issue, the barriers
+// of two or three short stages an item first among the stalls).
 
 #include "kernels.hpp"
 #include "smooth_line.cuh"
