@@ -10,7 +10,7 @@
 //                                                     of length n2 with the transposed store; the batch runs in
 //                                                     waves whose intermediate fits in L2 (the reference's Bailey
 //                                                     four-step, kernels/fft_kernels.cpp:2363-2658)
-//   n with a prime factor above 7                     Bluestein chirp-z over a power-of-two plan (bluestein.hpp)
+//   n with a prime factor above 7                     Bluestein chirp-z at a 7-smooth length (bluestein.hpp)
 //   R2C / C2R                                         half-length complex plan + recombine pass (real_fft.hpp)
 //   rank 2 / 3                                        one pass per axis, inverse by the conjugation trick
 //                                                     (nd_fft.hpp:105-147)

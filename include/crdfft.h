@@ -170,7 +170,7 @@ crdfft_status crdfft_rfft(crdfft_plan* plan, const float* real_in, void* out, vo
 crdfft_status crdfft_irfft(crdfft_plan* plan, const void* in, float* real_out, void* stream);
 
 /* BluesteinPlan<float>(alloc, n) (bluestein.hpp:31): any n >= 1; forward unnormalised, inverse normalised by 1/n.
- * 7-smooth n run natively in mixed radix; other n run the chirp-z algorithm over a power-of-two plan. */
+ * 7-smooth n run natively in mixed radix; other n run the chirp-z algorithm at a 7-smooth length >= 2n - 1. */
 crdfft_status crdfft_bluestein_plan_create(int64_t n, crdfft_plan** plan);
 /* BluesteinPlan::execute(data, dir) (bluestein.hpp:87-136): in place. */
 crdfft_status crdfft_bluestein_execute(crdfft_plan* plan, void* data, int32_t direction, void* stream);
