@@ -322,6 +322,16 @@ cudaError_t launch(const ChirpDesc& p, long long len, const void* tw, long long 
     return cudaGetLastError();
 }
 
+__global__ void chirp_gather_kernel(const float2* x, float2* w, long long n, long long dist, long long total)
+{
+    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
+         i += static_cast<long long>(gridDim.x) * blockDim.x)
+    {
+        const long long t = idiv(i, n);
+        w[i] = x[t * dist + (i - t * n)];
+    }
+}
+
 } // namespace
 } // namespace smooth
 
@@ -340,6 +350,15 @@ bool chirp_radices(long long m, std::vector<int>& out, double* arith)
                 out = {R / a, a};
     }
     return out.size() >= 2;
+}
+
+cudaError_t launch_chirp_gather(const ChirpDesc& p, const void* x, void* w, cudaStream_t stream)
+{
+    const long long total = p.n * p.batch;
+    const long long blocks = std::min((total + 255) / 256, 148LL * 8);
+    smooth::chirp_gather_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
+        static_cast<const float2*>(x), static_cast<float2*>(w), p.n, p.idist, total);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_chirp_line(const ChirpDesc& p, const void* x, void* out, cudaStream_t stream)

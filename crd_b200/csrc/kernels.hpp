@@ -150,6 +150,8 @@ struct ChirpDesc
 // The longest m one CTA transforms (two CTAs an SM); the radices of a convolution length (two or more stages), false when none.
 constexpr long long kChirpLine = 14000;
 bool chirp_radices(long long m, std::vector<int>& out, double* arith = nullptr);
+// The inputs, idist apart, side by side in w (for a call whose output overlaps them).
+cudaError_t launch_chirp_gather(const ChirpDesc& p, const void* x, void* w, cudaStream_t stream);
 cudaError_t launch_chirp_line(const ChirpDesc& p, const void* x, void* out, cudaStream_t stream);
 cudaError_t launch_chirp_cols_in(const ChirpDesc& p, const void* x, void* w, cudaStream_t stream);
 cudaError_t launch_chirp_rows(const ChirpDesc& p, void* w, cudaStream_t stream);

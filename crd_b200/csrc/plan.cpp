@@ -108,6 +108,7 @@ enum class StepKind : int
     Zero,
     R2CPost,
     C2RPre,
+    ChirpGather,
     ChirpLine,
     ChirpColsIn,
     ChirpRows,
@@ -418,6 +419,8 @@ struct Plan
     crdfft_desc desc{};
     int device = 0;
     std::vector<Step> steps[2];
+    // Chirp-z with unequal distances: the steps of a call whose input and output overlap (empty: steps serve it).
+    std::vector<Step> aliased[2];
     std::vector<void*> tables;
     std::map<std::vector<int>, void*> tw_by_radices;
     long long table_bytes = 0;
@@ -1840,7 +1843,6 @@ crdfft_status build_c2c_rank1(Plan& p)
     c.m = m;
     c.n1 = n1;
     c.n2 = n2;
-    c.idist = idist;
     c.odist = odist;
     void* dev = nullptr;
     crdfft_status st = upload_table(p, chirp, &dev);
@@ -1867,6 +1869,8 @@ crdfft_status build_c2c_rank1(Plan& p)
         if (st != CRDFFT_OK)
             return st;
     }
+    const long long padded = n1 == 0 ? 0 : wave * m;
+    const bool gather = idist != odist && B > 1;
     for (int dir = 0; dir < 2; ++dir)
     {
         c.conj = dir;
@@ -1874,29 +1878,47 @@ crdfft_status build_c2c_rank1(Plan& p)
         if (dir == 1 && d.norm == CRDFFT_NORM_INVERSE)
             sc /= static_cast<double>(n);
         c.scale = static_cast<float>(sc);
-        for (long long t0 = 0; t0 < B; t0 += wave)
-        {
-            c.batch = std::min(wave, B - t0);
-            const BufRef in{Buf::In, t0 * idist}, out{Buf::Out, t0 * odist}, ws{Buf::Ws, 0};
-            auto add = [&](StepKind kind, BufRef src, BufRef dst) {
-                Step s;
-                s.kind = kind;
-                s.chirp = c;
-                s.src = src;
-                s.dst = dst;
-                p.steps[dir].push_back(s);
-            };
-            if (n1 == 0)
-                add(StepKind::ChirpLine, in, out);
-            else
+        // The transforms of the batch, input `src` with `dist` between them.
+        auto transforms = [&](std::vector<Step>& steps, BufRef src, long long dist) {
+            c.idist = dist;
+            for (long long t0 = 0; t0 < B; t0 += wave)
             {
-                add(StepKind::ChirpColsIn, in, ws);
-                add(StepKind::ChirpRows, ws, ws);
-                add(StepKind::ChirpColsOut, ws, out);
+                c.batch = std::min(wave, B - t0);
+                const BufRef in{src.b, src.off + t0 * dist}, out{Buf::Out, t0 * odist}, ws{Buf::Ws, 0};
+                auto add = [&](StepKind kind, BufRef from, BufRef to) {
+                    Step s;
+                    s.kind = kind;
+                    s.chirp = c;
+                    s.src = from;
+                    s.dst = to;
+                    steps.push_back(s);
+                };
+                if (n1 == 0)
+                    add(StepKind::ChirpLine, in, out);
+                else
+                {
+                    add(StepKind::ChirpColsIn, in, ws);
+                    add(StepKind::ChirpRows, ws, ws);
+                    add(StepKind::ChirpColsOut, ws, out);
+                }
             }
-        }
+        };
+        transforms(p.steps[dir], BufRef{Buf::In, 0}, idist);
+        if (!gather)
+            continue;
+        // In place at unequal distances a transform's output covers inputs of others that are still to be read: the
+        // whole input moves to the workspace first.
+        Step g;
+        g.kind = StepKind::ChirpGather;
+        g.chirp = c;
+        g.chirp.batch = B;
+        g.chirp.idist = idist;
+        g.src = BufRef{Buf::In, 0};
+        g.dst = BufRef{Buf::Ws, padded};
+        p.aliased[dir].push_back(g);
+        transforms(p.aliased[dir], g.dst, n);
     }
-    p.ws_bytes = n1 == 0 ? 0 : static_cast<size_t>(wave * m) * 8;
+    p.ws_bytes = static_cast<size_t>(padded + (gather ? B * n : 0)) * 8;
     p.algorithm = "bluestein";
     p.factors = {n, m};
     return CRDFFT_OK;
@@ -3021,6 +3043,17 @@ crdfft_status run_uneven(Plan& p, const void* in, void* out, int dir, cudaStream
     return cudaGraphLaunch(exec, stream) == cudaSuccess ? CRDFFT_OK : CRDFFT_LAUNCH;
 }
 
+// Whether the rank-1 batch's input and output share memory.
+bool overlap(const crdfft_desc& d, const void* in, const void* out)
+{
+    const long long n = d.dims[0];
+    auto bytes = [&](long long dist) {
+        return static_cast<size_t>((d.batch - 1) * (dist ? dist : n) + n) * 8;
+    };
+    const auto a = reinterpret_cast<uintptr_t>(in), b = reinterpret_cast<uintptr_t>(out);
+    return a < b + bytes(d.odist) && b < a + bytes(d.idist);
+}
+
 crdfft_status run(Plan& p, const void* in, void* out, int dir, cudaStream_t stream, const void* spec = nullptr)
 {
     int dev = -1;
@@ -3047,7 +3080,8 @@ crdfft_status run(Plan& p, const void* in, void* out, int dir, cudaStream_t stre
         forked = false;
         return true;
     };
-    for (const Step& s : p.steps[dir])
+    const bool aliased = !p.aliased[dir].empty() && overlap(p.desc, in, out);
+    for (const Step& s : aliased ? p.aliased[dir] : p.steps[dir])
     {
         if (s.lane != 0)
         {
@@ -3102,6 +3136,7 @@ crdfft_status run(Plan& p, const void* in, void* out, int dir, cudaStream_t stre
                 break;
             case StepKind::R2CPost: e = launch_r2c_post(s.real, src, dst, stream); break;
             case StepKind::C2RPre: e = launch_c2r_pre(s.real, src, dst, stream); break;
+            case StepKind::ChirpGather: e = launch_chirp_gather(s.chirp, src, dst, stream); break;
             case StepKind::ChirpLine: e = launch_chirp_line(s.chirp, src, dst, stream); break;
             case StepKind::ChirpColsIn: e = launch_chirp_cols_in(s.chirp, src, dst, stream); break;
             case StepKind::ChirpRows: e = launch_chirp_rows(s.chirp, dst, stream); break;

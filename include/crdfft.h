@@ -114,7 +114,8 @@ crdfft_status crdfft_plan_create(const crdfft_desc* desc, crdfft_plan** plan);
 /* Release a plan, its tables and its owned workspace. NULL is accepted. */
 crdfft_status crdfft_plan_destroy(crdfft_plan* plan);
 
-/* Run the plan: `in` -> `out` (in == out allowed for C2C, the reference's in-place execute, fft.hpp:409-413).
+/* Run the plan: `in` -> `out` (in == out allowed for C2C, the reference's in-place execute, fft.hpp:409-413, where
+ * input and output have the same strides and distances; lengths with a prime factor above 7 take any distances).
  * `direction` is crdfft_direction; R2C plans accept only CRDFFT_FORWARD and C2R plans only CRDFFT_INVERSE. */
 crdfft_status crdfft_execute(crdfft_plan* plan, const void* in, void* out, int32_t direction, void* stream);
 

@@ -52,3 +52,26 @@ def test_padded_leaves_the_gaps(dev, n):
     got = out.cpu().numpy()
     assert oracle.rel_l2(got[:, :n], np.fft.fft(x[:, :n].astype(np.complex128))) <= 1e-6
     assert np.all(got[:, n:] == 9.0)
+
+
+@pytest.mark.parametrize("n,batch", [(11, 2), (101, 1000), (6997, 40), (10007, 301)])
+@pytest.mark.parametrize("gaps", [(0, 3), (5, 0)])
+@pytest.mark.parametrize("shift", [0, 7])
+def test_in_place_at_unequal_distances(dev, n, batch, gaps, shift):
+    """Input and output in one buffer with other distances (and, shifted, another start): every transform's input is read
+    before any output covers it, so the result is the out-of-place call's, whose gaps the call leaves alone."""
+    import torch
+
+    import crd_b200 as cf
+
+    idist, odist = n + gaps[0], n + gaps[1]
+    plan = cf.Plan([n], batch=batch, idist=idist, odist=odist, norm=cf.NORM_INVERSE)
+    size = shift + batch * max(idist, odist)
+    buf = torch.from_numpy(oracle.lcg_complex64(n + shift, size)).cuda()
+    for direction in (cf.FORWARD, cf.INVERSE):
+        want = buf.clone()
+        plan.execute(buf, want[shift:], direction)
+        both = buf.clone()
+        plan.execute(both, both[shift:], direction)
+        torch.cuda.synchronize()
+        assert torch.equal(both, want)
