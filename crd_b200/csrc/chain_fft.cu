@@ -23,10 +23,11 @@
 #include "chain_list.hpp"
 #include "kernels.hpp"
 #include "line_fft.cuh"
+#include "smem_limit.hpp"
 #include "smooth_line.cuh"
 #include "smooth_plan.hpp"
 
-#include <mutex>
+#include <type_traits>
 
 namespace crdfft
 {
@@ -207,13 +208,8 @@ cudaError_t launch_chain(const ChainDesc& cd, const void* in, void* out, void* w
     if (a < 0 || b < 0)
         return cudaErrorInvalidConfiguration;
     const int smem = a > b ? a : b;
-    static std::mutex mu;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     const long long total = chain_list_length(cd.waves, cd.col_items, cd.row_items, cd.lag);
     if (total >= 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;

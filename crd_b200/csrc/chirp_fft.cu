@@ -14,6 +14,7 @@
 
 #include "kernels.hpp"
 #include "pass_desc.hpp"
+#include "smem_limit.hpp"
 #include "smooth_line.cuh"
 #include "smooth_plan.hpp"
 
@@ -292,12 +293,8 @@ cudaError_t launch(const ChirpDesc& p, long long len, const void* tw, long long 
         return cudaErrorInvalidConfiguration;
     const bool wide = smooth_wide(rad.data(), static_cast<int>(rad.size()));
     const auto fn = wide ? chirp_kernel<PASS, true> : chirp_kernel<PASS, false>;
-    if (smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     // Full column tiles take up to 256 threads, the most that leave the fewest idle in the stages' last rounds: fewer,
     // larger CTAs, since warps of one CTA are in the same stage and share its instructions (128-point columns, 32 a
     // tile: 10007 x 251 in 90.3 us with 256, 95.8 with 128; 168 points in 60 us with 160 or 192, 70 with 256).

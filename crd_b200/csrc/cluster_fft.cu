@@ -16,6 +16,7 @@
 
 #include "kernels.hpp"
 #include "line_fft.cuh"
+#include "smem_limit.hpp"
 
 #include <cooperative_groups.h>
 
@@ -202,12 +203,8 @@ cudaError_t launch_cluster_fft(const PassDesc& a, const PassDesc& b, long long b
     // The four-step twiddle is applied in the exchange, so only conjugation and scale select the EPI instance.
     const bool epi = a.conj_in != 0 || b.conj_out != 0 || b.scale != 1.0f;
     lfft::ClusterFn fn = epi ? e->fn_epi : e->fn_plain;
-    if (e->smem_bytes > 48 * 1024)
-    {
-        const cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, e->smem_bytes);
-        if (err != cudaSuccess)
-            return err;
-    }
+    if (const cudaError_t err = allow_smem(fn, e->smem_bytes); err != cudaSuccess)
+        return err;
     const long long grid = batch * e->cluster;
     if (grid > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;

@@ -14,6 +14,7 @@
 #include "kernels.hpp"
 #include "line_fft.cuh"
 #include "real_pair.cuh"
+#include "smem_limit.hpp"
 
 namespace crdfft
 {
@@ -399,12 +400,8 @@ cudaError_t launch_conv(const PassDesc& d, PassMap map, const LineMap& smap, con
         return cudaSuccess;
     if (groups > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    if (smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     fn<<<static_cast<unsigned>(groups), T * lpc, smem, stream>>>(d, static_cast<const float2*>(in),
                                                                  static_cast<const float2*>(spec), smap,
                                                                  static_cast<float2*>(out));
@@ -432,12 +429,8 @@ cudaError_t launch_cwt_lines(const PassDesc& d, const void* X, const void* K, co
         return cudaSuccess;
     if (groups > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    if (smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     fn<<<static_cast<unsigned>(groups), T * lpc, smem, stream>>>(
         d, static_cast<const float2*>(X), static_cast<const float2*>(K), scales, nscales, n,
         static_cast<float>(1.0 / static_cast<double>(d.n)), static_cast<float2*>(out));
@@ -466,12 +459,8 @@ cudaError_t launch_cwt_real_lines(const PassDesc& d, const void* X, const void* 
         return cudaSuccess;
     if (groups > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    if (smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     fn<<<static_cast<unsigned>(groups), T * lpc, smem, stream>>>(
         d, static_cast<const float2*>(X), static_cast<const float2*>(K), static_cast<const float2*>(wn), scales, nscales,
         n, static_cast<float>(0.5 / static_cast<double>(d.n)), static_cast<float2*>(out));

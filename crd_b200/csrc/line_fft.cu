@@ -3,6 +3,7 @@
 
 #include "kernels.hpp"
 #include "line_fft.cuh"
+#include "smem_limit.hpp"
 
 #include <mutex>
 #include <unordered_map>
@@ -168,12 +169,8 @@ cudaError_t launch_line_pass(const PassDesc& d, const PassShape& sh, const void*
         lfft::PipeFn fn = lfft::select_pipe(d, sh);
         if (fn == nullptr || threads > lfft::kPipeThreads)
             return cudaErrorInvalidConfiguration;
-        if (sh.smem_bytes > 48 * 1024)
-        {
-            const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem_bytes);
-            if (e != cudaSuccess)
-                return e;
-        }
+        if (const cudaError_t e = allow_smem(fn, sh.smem_bytes); e != cudaSuccess)
+            return e;
         const long long cap = static_cast<long long>(sm_count()) *
                               resident_ctas(reinterpret_cast<const void*>(fn), threads, sh.smem_bytes);
         const long long grid = groups < cap ? groups : cap;
@@ -196,12 +193,8 @@ cudaError_t launch_line_pass(const PassDesc& d, const PassShape& sh, const void*
         return cudaErrorInvalidConfiguration;
     if (groups > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    if (cs.smem_bytes > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, cs.smem_bytes);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, cs.smem_bytes); e != cudaSuccess)
+        return e;
     fn<<<static_cast<unsigned>(groups), threads, cs.smem_bytes, stream>>>(d, static_cast<const float2*>(in),
                                                                            static_cast<float2*>(out));
     return cudaGetLastError();

@@ -20,6 +20,7 @@
 #include "kernels.hpp"
 #include "line_fft.cuh"
 #include "real_pair.cuh"
+#include "smem_limit.hpp"
 
 namespace crdfft
 {
@@ -401,12 +402,8 @@ cudaError_t launch_row_r2c(const PassDesc& row, const RowR2CDesc& r, const void*
         return cudaSuccess;
     if (blocks > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    if (smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     fn<<<static_cast<unsigned>(blocks), threads, smem, stream>>>(row, r, static_cast<const float2*>(ws),
                                                                  static_cast<float2*>(out));
     return cudaGetLastError();
@@ -436,12 +433,8 @@ cudaError_t launch_real_line(const PassDesc& d, int mode, const RealLineAux& r, 
         return cudaSuccess;
     if (groups > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    if (smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     fn<<<static_cast<unsigned>(groups), T * lpc, smem, stream>>>(d, static_cast<const float2*>(in),
                                                                  static_cast<const float2*>(spec), r,
                                                                  static_cast<float2*>(out));

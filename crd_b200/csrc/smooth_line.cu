@@ -5,6 +5,7 @@
 #include "index.cuh"
 #include "kernels.hpp"
 #include "pass_desc.hpp"
+#include "smem_limit.hpp"
 #include "smooth_line.cuh"
 #include "smooth_plan.hpp"
 
@@ -269,12 +270,8 @@ cudaError_t launch_smooth_line(const PassDesc& d, int lpc, const void* in, void*
                           {smooth::smooth_line_kernel<0, true>, smooth::smooth_line_kernel<1, true>,
                            smooth::smooth_line_kernel<2, true>}};
     const Fn fn = fns[wide ? 1 : 0][epi];
-    if (smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     fn<<<static_cast<unsigned>(groups), smooth_threads(s, lpc, smem, regs, groups), smem, stream>>>(
         d, s, smooth::tile_of(d, s, lpc), static_cast<const float2*>(in), static_cast<float2*>(out));
     return cudaGetLastError();

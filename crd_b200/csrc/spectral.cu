@@ -17,6 +17,7 @@
 #include "kernels.hpp"
 #include "line_fft.cuh"
 #include "real_pair.cuh"
+#include "smem_limit.hpp"
 
 namespace crdfft
 {
@@ -336,12 +337,8 @@ cudaError_t launch_spectral(const PassDesc& d, const SpectralDesc& sd, int threa
         return cudaSuccess;
     if (blocks > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    if (smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     fn<<<static_cast<unsigned>(blocks), threads, smem, stream>>>(d, sd, static_cast<const float*>(x),
                                                                  static_cast<float*>(out));
     return cudaGetLastError();

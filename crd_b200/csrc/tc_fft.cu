@@ -27,6 +27,7 @@
 
 #include "kernels.hpp"
 #include "line_fft.cuh"
+#include "smem_limit.hpp"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -422,7 +423,7 @@ cudaError_t launch_tc_pass(const PassDesc& d, int prec, const void* amat, const 
     if (fn == nullptr)
         return cudaErrorInvalidConfiguration;
     const int smem = lfft::tc_smem_bytes(d.n, prec);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem(fn, smem);
     if (e != cudaSuccess)
         return e;
     const int lpc = lfft::kTcCols / (d.n / 16);

@@ -23,6 +23,7 @@
 
 #include "kernels.hpp"
 #include "line_fft.cuh"
+#include "smem_limit.hpp"
 
 namespace crdfft
 {
@@ -368,8 +369,7 @@ cudaError_t launch_tma_col(const PassDesc& d, const void* in, void* out, cudaStr
     if (nbuf < 2)
         return cudaErrorInvalidConfiguration;
     const int smem = 1024 + nbuf * tile_stride + nbuf * 8 + 16;
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess)
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
         return e;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -425,12 +425,8 @@ cudaError_t launch_row_tstore(const PassDesc& d, const PassShape& sh, const void
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue; // the tensor map was refused
     const int smem = 1024 + lpc * lfft::cta_line_pitch(d.n, lpc) * 8;
-    if (smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
+        return e;
     const long long grid = d.lines / lpc;
     if (grid > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;

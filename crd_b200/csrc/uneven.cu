@@ -26,6 +26,7 @@
 // of two or three short stages an item first among the stalls).
 
 #include "kernels.hpp"
+#include "smem_limit.hpp"
 #include "smooth_line.cuh"
 #include "uneven.hpp"
 
@@ -216,8 +217,7 @@ __global__ void __launch_bounds__(kThreads, 3)
 
 int uneven_resident(int smem_bytes)
 {
-    if (smem_bytes > 48 * 1024 && cudaFuncSetAttribute(smooth::uneven_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       smem_bytes) != cudaSuccess)
+    if (allow_smem(smooth::uneven_kernel, smem_bytes) != cudaSuccess)
         return 0;
     int per_sm = 0, dev = 0, sms = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, smooth::uneven_kernel, smooth::kThreads, smem_bytes) !=

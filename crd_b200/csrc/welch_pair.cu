@@ -14,6 +14,7 @@
 #include "codelets.cuh"
 #include "index.cuh"
 #include "kernels.hpp"
+#include "smem_limit.hpp"
 
 #include <algorithm>
 #include <vector>
@@ -249,12 +250,8 @@ cudaError_t launch_welch_pair(const SpectralDesc& sd, const void* x, void* part,
         return cudaSuccess;
     if (blocks > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    if (p->smem > 48 * 1024)
-    {
-        const cudaError_t e = cudaFuncSetAttribute(p->fn, cudaFuncAttributeMaxDynamicSharedMemorySize, p->smem);
-        if (e != cudaSuccess)
-            return e;
-    }
+    if (const cudaError_t e = allow_smem(p->fn, p->smem); e != cudaSuccess)
+        return e;
     p->fn<<<static_cast<unsigned>(blocks), p->threads, p->smem, stream>>>(sd, static_cast<const float*>(x),
                                                                           static_cast<float*>(part));
     return cudaGetLastError();
