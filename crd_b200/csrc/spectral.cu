@@ -231,18 +231,18 @@ __global__ void __launch_bounds__(DYN ? kMaxThreads : kStaticThreads, DYN ? 1 : 
     }
 }
 
-// The per-CTA sums of each signal added in a fixed order, divided by the segment count (spectral.hpp:158-171): eight
-// slices of consecutive rows, each in row order, then the slices in order (one thread over all the rows of a frequency
-// took 58 us for 16 signals x 1024 rows of 513).
-constexpr int kFinishFreqs = 32;
-constexpr int kFinishSlices = 8;
-__global__ void __launch_bounds__(kFinishFreqs* kFinishSlices)
+// The per-CTA sums of each signal added in a fixed order, divided by the segment count (spectral.hpp:158-171): `slices`
+// of consecutive rows, each in row order, then the slices in order (finish_slices).
+constexpr int kFinishThreads = 256;
+__global__ void __launch_bounds__(kFinishThreads)
     welch_finish_kernel(const float* __restrict__ part, float* __restrict__ psd, long long count, int ntiles, int nfreq,
-                        float nseg)
+                        float nseg, int slices)
 {
-    __shared__ float sums[kFinishSlices][kFinishFreqs];
-    const long long idx = static_cast<long long>(blockIdx.x) * kFinishFreqs + threadIdx.x % kFinishFreqs;
-    const int slice = threadIdx.x / kFinishFreqs;
+    __shared__ float sums[kFinishThreads];
+    const int freqs = kFinishThreads / slices; // a CTA's frequencies
+    const int slice = threadIdx.x / freqs;
+    const int k0 = threadIdx.x - slice * freqs;
+    const long long idx = static_cast<long long>(blockIdx.x) * freqs + k0;
     const bool ok = idx < count * nfreq;
     float acc = 0.0f;
     if (ok)
@@ -250,18 +250,29 @@ __global__ void __launch_bounds__(kFinishFreqs* kFinishSlices)
         const long long g = idiv(idx, nfreq);
         const int k = static_cast<int>(idx - g * nfreq);
         const float* p = part + g * ntiles * static_cast<long long>(nfreq) + k;
-        const int each = (ntiles + kFinishSlices - 1) / kFinishSlices;
+        const int each = (ntiles + slices - 1) / slices;
         const int end = min(ntiles, (slice + 1) * each);
         for (int t = slice * each; t < end; ++t)
             acc += p[static_cast<long long>(t) * nfreq];
     }
-    sums[slice][threadIdx.x % kFinishFreqs] = acc;
+    sums[threadIdx.x] = acc;
     __syncthreads();
     if (slice != 0 || !ok)
         return;
-    for (int s = 1; s < kFinishSlices; ++s)
-        acc += sums[s][threadIdx.x];
+    for (int s = 1; s < slices; ++s)
+        acc += sums[s * freqs + k0];
     psd[idx] = acc / nseg;
+}
+
+// Slices of a signal's rows: as many, up to eight of four rows or more, as fill the device (148 x 2048 threads) when the
+// frequencies alone do not: 16 signals x 1024 rows of 513 took 58 us as one slice, most of the device idle; 2000 signals
+// x 1 row of 2049 took 248 us with the transforms when every row had eight slices, seven of them empty, and take 86.
+int finish_slices(long long freqs, int ntiles)
+{
+    int s = 1;
+    while (s < 8 && ntiles >= 8 * s && freqs * s < 148LL * 2048)
+        s *= 2;
+    return s;
 }
 
 using SpecFn = void (*)(const PassDesc, const SpectralDesc, const float*, float*);
@@ -350,12 +361,14 @@ cudaError_t launch_welch_finish(const SpectralDesc& sd, const void* part, void* 
     const long long total = sd.count * nfreq;
     if (total <= 0)
         return cudaSuccess;
-    const long long blocks = (total + lfft::kFinishFreqs - 1) / lfft::kFinishFreqs;
+    const int slices = lfft::finish_slices(total, sd.ntiles);
+    const long long freqs = lfft::kFinishThreads / slices;
+    const long long blocks = (total + freqs - 1) / freqs;
     if (blocks > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
-    lfft::welch_finish_kernel<<<static_cast<unsigned>(blocks), lfft::kFinishFreqs * lfft::kFinishSlices, 0, stream>>>(
+    lfft::welch_finish_kernel<<<static_cast<unsigned>(blocks), lfft::kFinishThreads, 0, stream>>>(
         static_cast<const float*>(part), static_cast<float*>(psd), sd.count, sd.ntiles, nfreq,
-        static_cast<float>(sd.nseg));
+        static_cast<float>(sd.nseg), slices);
     return cudaGetLastError();
 }
 

@@ -55,3 +55,14 @@ def test_loud_beside_quiet(dev):
     x = np.random.default_rng(4).uniform(-1, 1, (1, 64 * 512)).astype(np.float32)
     x[0, : 512 * 8] *= 1000.0
     check(run(x, 512, 1), x, 512, 1)
+
+
+@pytest.mark.parametrize("nperseg,nseg,count", [(4096, 3, 300), (1000, 16, 640), (1000, 33, 400), (1000, 70, 100),
+                                                (128, 600, 9), (256, 1, 2500)])
+def test_sums_of_few_and_many_rows(dev, nperseg, nseg, count):
+    """Few and many rows of sums a signal under few and many frequencies: one to eight slices of rows."""
+    n = nperseg + (nseg - 1) * (nperseg // 2)
+    x = np.random.default_rng(nseg).uniform(-1, 1, (count, n)).astype(np.float32)
+    got = run(x, nperseg)
+    keep = sorted({0, 1, count // 2, count - 1})
+    check(got[keep], x[keep], nperseg)
