@@ -2848,6 +2848,20 @@ crdfft_status build_spectral(Plan& p, const crdfft_spectral_desc& s)
     }
     if (!(ss > 0.0))
         return CRDFFT_INVALID_ARG;
+    const bool welch = s.mode == CRDFFT_SPECTRAL_WELCH;
+    double scale = 1.0 / (s.fs * ss);
+    std::vector<int> pair_rad;
+    int pair_tiles = 0, pairs_cta = 0;
+    if (welch && g.nseg > 0 && welch_pair_shape(static_cast<int>(n), s.count, g.nseg, &pair_rad, &pair_tiles, &pairs_cta) &&
+        std::isfinite(scale))
+    {
+        // The pair kernel sums powers before it scales them: a power of two near the root of the scale goes into its
+        // window, exactly, which leaves a factor in [1, 4) for the end, so no sum overflows before its scaled value does.
+        const int e = std::clamp(static_cast<int>(std::floor(std::log2(scale) / 2.0)), -60, 60);
+        for (float& w : win)
+            w = std::ldexp(w, e);
+        scale = std::ldexp(scale, -2 * e);
+    }
     void* dwin = nullptr;
     crdfft_status st = upload_table(p, win, &dwin);
     if (st != CRDFFT_OK)
@@ -2866,7 +2880,6 @@ crdfft_status build_spectral(Plan& p, const crdfft_spectral_desc& s)
         return st;
     p.spectral = true;
     p.factors = {n, g.nseg};
-    const bool welch = s.mode == CRDFFT_SPECTRAL_WELCH;
     p.algorithm = welch ? "spectral-welch" : s.mode == CRDFFT_SPECTRAL_SPECTROGRAM ? "spectral-spectrogram"
                                                                                     : "spectral-periodogram";
     if (g.nseg == 0)
@@ -2900,13 +2913,14 @@ crdfft_status build_spectral(Plan& p, const crdfft_spectral_desc& s)
     sd.ntiles = static_cast<int>((g.nseg + lpc - 1) / lpc);
     sd.detrend = s.detrend ? 1 : 0;
     sd.welch = welch ? 1 : 0;
-    sd.scale = static_cast<float>(1.0 / (s.fs * ss));
+    sd.scale = static_cast<float>(scale);
     sd.win = static_cast<const float*>(dwin);
     sd.wn = dwn;
-    std::vector<int> rad;
-    if (welch && welch_pair_shape(sd.nperseg, sd.count, sd.nseg, &rad, &sd.ntiles, &sd.ppc))
+    if (!pair_rad.empty())
     {
-        st = twiddle_table(p, rad, &sd.pair_tw);
+        sd.ntiles = pair_tiles;
+        sd.ppc = pairs_cta;
+        st = twiddle_table(p, pair_rad, &sd.pair_tw);
         if (st != CRDFFT_OK)
             return st;
     }

@@ -66,3 +66,18 @@ def test_sums_of_few_and_many_rows(dev, nperseg, nseg, count):
     got = run(x, nperseg)
     keep = sorted({0, 1, count // 2, count - 1})
     check(got[keep], x[keep], nperseg)
+
+
+@pytest.mark.parametrize("nperseg", [256, 1024, 4096])
+@pytest.mark.parametrize("amplitude,fs", [(None, 1.0), (1e-10, 1e-12), (1e12, 1e14), (1e-14, 1e6)])
+def test_range(dev, nperseg, amplitude, fs):
+    """The sums hold scaled powers, as the definition's do. None: each segment's power is half the FP32 maximum, and the
+    sum of 24 fits after the density's scale only; the others have scales far from 1 either way."""
+    count, n = 8, nperseg // 2 * 25
+    if amplitude is None:
+        amplitude = 5e19 / nperseg  # a Hann-windowed tone of amplitude A has the power (A nperseg / 4)^2 = 1.6e38
+    x = np.random.default_rng(5).uniform(-0.1, 0.1, (count, n)) + np.cos(2 * np.pi * 5 / 64 * np.arange(n))
+    x = (amplitude * x).astype(np.float32)
+    got = run(x, nperseg, fs=fs)
+    assert np.all(np.isfinite(got))
+    check(got[:2], x[:2], nperseg, fs=fs)
