@@ -263,14 +263,14 @@ __global__ void __launch_bounds__(256, P == 16 ? 4 : 2)
     {
         const CwtScale p = scales[s];
         float2* o = gout + line * nsamples;
-        auto w = [&](int t) {
+        auto w = [&](int t) { // already the difference of two filtered samples: K's kernels are differences
             const float2* e = &lay.at(t >> 1);
             return (t & 1) ? -e->y : e->x;
         };
         const float g = p.taps_ok ? p.amp * inv_n : 0.0f;
         const int off = p.taps_ok ? static_cast<int>(p.off) : 0;
         for (int i = jt; i < static_cast<int>(nsamples); i += T)
-            __stcs(o + i, make_float2(p.taps_ok ? g * (w(off + i + 1) - w(off + i)) : 0.0f, 0.0f));
+            __stcs(o + i, make_float2(p.taps_ok ? g * w(off + i) : 0.0f, 0.0f));
     }
 }
 

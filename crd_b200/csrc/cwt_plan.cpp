@@ -390,7 +390,7 @@ crdfft_status build(const crdfft_cwt_desc* d, const Geometry& g, crdfft_cwt_plan
     if (cudaGetDevice(&p->device) != cudaSuccess)
         return CRDFFT_NO_DEVICE;
 
-    // the integrated wavelet (cwt.hpp:470-477), each scale's reversed kernel narrowed to FP32 (cwt.hpp:569-581)
+    // the integrated wavelet (cwt.hpp:470-477)
     std::vector<cd> ipsi = sample_psi(g.w, g.grid_n);
     cd acc(0.0, 0.0);
     for (cd& v : ipsi)
@@ -398,30 +398,6 @@ crdfft_status build(const crdfft_cwt_desc* d, const Geometry& g, crdfft_cwt_plan
         acc += v;
         v = g.w.complex_valued ? std::conj(acc * g.step) : acc * g.step;
     }
-    std::vector<float> table(static_cast<size_t>(ns * lfft) * 2, 0.0f);
-    std::vector<crdfft::CwtScale> sc(static_cast<size_t>(ns));
-    for (long long s = 0; s < ns; ++s)
-    {
-        const double a = d->scales[s];
-        const long long kk = g.taps[static_cast<size_t>(s)];
-        crdfft::CwtScale& c = sc[static_cast<size_t>(s)];
-        c.taps_ok = kk >= 2 ? 1 : 0;
-        c.off = kk >= 2 ? (kk - 2) / 2 : 0;
-        c.amp = -static_cast<float>(std::sqrt(a));
-        if (c.off + d->nsamples >= lfft)
-            return CRDFFT_INVALID_DESC; // cannot happen: lfft >= n + kk
-        if (kk < 2)
-            continue;
-        float* row = table.data() + static_cast<size_t>(s * lfft) * 2;
-        for (long long i = 0; i < kk; ++i)
-        {
-            const long long m = kk - 1 - i;
-            const cd v = ipsi[static_cast<size_t>(static_cast<double>(m) / (a * g.step))];
-            row[2 * i] = static_cast<float>(v.real());
-            row[2 * i + 1] = static_cast<float>(v.imag());
-        }
-    }
-
     // the fused line kernel where the FFT length has a compile-time schedule: one launch, no filtered-sequence scratch
     const long long line_bytes = lfft * 8;
     crdfft_desc ld = line_desc(lfft, d->count * ns);
@@ -466,6 +442,42 @@ crdfft_status build(const crdfft_cwt_desc* d, const Geometry& g, crdfft_cwt_plan
             p->lines_plan = nullptr;
         }
     }
+    // Each scale's reversed kernel narrowed to FP32 (cwt.hpp:569-581). For the half-length lines its differences
+    // h[i + 1] - h[i], i >= -1, at i mod lfft: a coefficient is the difference of two neighbouring filtered samples
+    // (cwt.hpp:589-596), and filtering with the differences, taken in FP64, gives it without the cancellation that
+    // magnifies an FP32 transform's rounding (64 scales to 128 of 64 signals x 4096: rel-L2 1.9e-7, 1.6e-6 for morl and
+    // 5.9e-6 for mexh when the filtered samples are subtracted).
+    std::vector<float> table(static_cast<size_t>(ns * lfft) * 2, 0.0f);
+    std::vector<crdfft::CwtScale> sc(static_cast<size_t>(ns));
+    for (long long s = 0; s < ns; ++s)
+    {
+        const double a = d->scales[s];
+        const long long kk = g.taps[static_cast<size_t>(s)];
+        crdfft::CwtScale& c = sc[static_cast<size_t>(s)];
+        c.taps_ok = kk >= 2 ? 1 : 0;
+        c.off = kk >= 2 ? (kk - 2) / 2 : 0;
+        c.amp = -static_cast<float>(std::sqrt(a));
+        if (c.off + d->nsamples >= lfft)
+            return CRDFFT_INVALID_DESC; // cannot happen: lfft >= n + kk
+        if (kk < 2)
+            continue;
+        float* row = table.data() + static_cast<size_t>(s * lfft) * 2;
+        auto tap = [&](long long i) { // the reversed kernel, zero beyond its taps
+            const long long m = kk - 1 - i;
+            return i < 0 || i >= kk ? cd(0.0, 0.0) : ipsi[static_cast<size_t>(static_cast<double>(m) / (a * g.step))];
+        };
+        cd last(0.0, 0.0);
+        for (long long i = p->real_lines ? -1 : 0; i < kk; ++i)
+        {
+            const cd h = tap(p->real_lines ? i + 1 : i);
+            const cd v = p->real_lines ? h - last : h;
+            const long long at = i < 0 ? lfft - 1 : i;
+            last = h;
+            row[2 * at] = static_cast<float>(v.real());
+            row[2 * at + 1] = static_cast<float>(v.imag());
+        }
+    }
+
     // otherwise signals a round: the filtered sequences within 512 MiB, the grid rows (lines) within 65535
     p->chunk = p->fused ? d->count
                         : std::max<long long>(1, std::min<long long>({static_cast<long long>(d->count),

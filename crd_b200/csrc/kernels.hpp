@@ -81,7 +81,7 @@ struct SpectralDesc
     int ntiles;         // CTAs a signal
     int detrend;        // subtract each segment's mean
     int welch;
-    float scale;        // 1 / (fs sum w^2)
+    float scale;        // 1 / (fs sum w^2); with pairs, over a power of two that win's values carry the root of
     const float* win;   // nperseg window values
     const void* wn;     // float2 W_nperseg^k, k = 0 .. M/2 at least
     int ppc;            // segment pairs a CTA (welch_pair.cu); 0: the segment-by-segment kernel
@@ -203,8 +203,8 @@ cudaError_t launch_cwt_diff(const void* W, const CwtScale* scales, void* out, lo
 // d.lines = signals x nscales lines of this launch. cwt_lines_supported: a compile-time schedule exists for d.
 bool conv_line_pass(crdfft_plan* plan, PassDesc* out);
 bool cwt_lines_supported(const PassDesc& d);
-// For a real wavelet (X and K then spectra of real sequences, 2 d.n values a line): d is the half-length line, wn holds
-// W_{2 d.n}^k for k <= d.n / 2.
+// For a real wavelet (X and K then spectra of real sequences, 2 d.n values a line; K's are the kernels' differences): d is
+// the half-length line, wn holds W_{2 d.n}^k for k <= d.n / 2.
 bool cwt_real_lines_supported(const PassDesc& d);
 cudaError_t launch_cwt_real_lines(const PassDesc& d, const void* X, const void* K, const void* wn,
                                   const CwtScale* scales, long long nscales, long long n, void* out,
