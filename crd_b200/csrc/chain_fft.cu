@@ -55,18 +55,18 @@ __device__ __forceinline__ bool wait_at_least(const int* p, int target, int limi
     return false;
 }
 
-// A side without a compile-time schedule runs the run-time-schedule tile (smooth_line.cuh).
+// Columns without a compile-time schedule run the run-time-schedule tile (smooth_line.cuh), the build without the radices
+// above 16: this launch is the slower form (off by default), and six instances with them took three minutes to compile.
 using Smooth = void;
-struct SmoothSides
+struct SmoothSide
 {
-    SmoothSched col_s, row_s;
-    smooth::Tile col_t, row_t;
+    SmoothSched s;
+    smooth::Tile t;
 };
 
 template <class SC, int PC, class SR, int PR, bool REPI>
-__global__ void __maxnreg__((std::is_void_v<SC> || std::is_void_v<SR>) ? 96 : 80)
-    chain_fft_kernel(const ChainDesc cd, const SmoothSides sides, const float2* __restrict__ src,
-                     float2* __restrict__ dst, float2* ws)
+__global__ void __maxnreg__(80) chain_fft_kernel(const ChainDesc cd, const SmoothSide col,
+                                                 const float2* __restrict__ src, float2* __restrict__ dst, float2* ws)
 {
     __shared__ int s_item, s_ok;
     const int tid = threadIdx.x;
@@ -107,21 +107,14 @@ __global__ void __maxnreg__((std::is_void_v<SC> || std::is_void_v<SR>) ? 96 : 80
         if (is_col)
         {
             if constexpr (std::is_void_v<SC>)
-                smooth::pass_tile<2, true>(cd.col, sides.col_s, sides.col_t, src + t0 * cd.idist, slot, idx,
-                                           wt * cd.row.n);
+                smooth::pass_tile<2, false>(cd.col, col.s, col.t, src + t0 * cd.idist, slot, idx, wt * cd.row.n);
             else
                 lfft::line_fft_tile<SC, PC, PassMap::Col, true, true, true>(cd.col, src + t0 * cd.idist, slot, idx,
                                                                             cd.col_lpc, wt * cd.row.n, tid);
         }
         else
-        {
-            if constexpr (std::is_void_v<SR>)
-                smooth::pass_tile<REPI ? 1 : 0, true>(cd.row, sides.row_s, sides.row_t, slot, dst + t0 * cd.odist,
-                                                      idx, wt * cd.col.n);
-            else
-                lfft::line_fft_tile<SR, PR, PassMap::Row, true, false, REPI>(cd.row, slot, dst + t0 * cd.odist, idx,
-                                                                             cd.row_lpc, wt * cd.col.n, tid);
-        }
+            lfft::line_fft_tile<SR, PR, PassMap::Row, true, false, REPI>(cd.row, slot, dst + t0 * cd.odist, idx,
+                                                                         cd.row_lpc, wt * cd.col.n, tid);
     }
     // Every thread's stores of the tile are issued; one release makes them visible before the tile's signal.
     __syncthreads();
@@ -132,7 +125,7 @@ __global__ void __maxnreg__((std::is_void_v<SC> || std::is_void_v<SR>) ? 96 : 80
     }
 }
 
-using ChainFn = void (*)(const ChainDesc, const SmoothSides, const float2*, float2*, float2*);
+using ChainFn = void (*)(const ChainDesc, const SmoothSide, const float2*, float2*, float2*);
 
 template <class SC, int PC, class SR, int PR> ChainFn pick(bool repi)
 {
@@ -145,7 +138,10 @@ bool radices_are(const PassDesc& d, std::initializer_list<int> rs)
 }
 
 bool is_static(const PassDesc& d) { return pass_has_static(d, 16) || pass_has_static(d, 32); }
-bool is_smooth(const PassDesc& d) { return !is_static(d) && smooth_line_supported(d); }
+bool is_smooth(const PassDesc& d)
+{
+    return !is_static(d) && smooth_line_supported(d) && !smooth_wide(d.radix, d.nstages);
+}
 
 // The column / row schedule pairs with a chained instance (points a thread 16 on the compile-time sides).
 ChainFn select(const PassDesc& col, const PassDesc& row)
@@ -153,12 +149,8 @@ ChainFn select(const PassDesc& col, const PassDesc& row)
     const bool repi = lfft::pass_epi(row);
     if (is_smooth(col))
     {
-        if (is_smooth(row))
-            return pick<Smooth, 0, Smooth, 0>(repi);
-        if (radices_are(row, {16, 16, 4}))
-            return pick<Smooth, 0, Sched<16, 16, 4>, 16>(repi);
         if (radices_are(row, {16, 8, 4}))
-            return pick<Smooth, 0, Sched<16, 8, 4>, 16>(repi);
+            return pick<Smooth, 0, Sched<16, 8, 4>, 16>(repi); // 107520 = 210 x 512
         return nullptr;
     }
     if (radices_are(row, {16, 16, 4}))
@@ -189,7 +181,7 @@ bool chain_supported(const PassDesc& col, const PassDesc& row)
 
 int chain_lines(const PassDesc& d, PassMap map)
 {
-    return is_smooth(d) ? smooth_line_lpc(d, map) : chain_lines_per_tile(d.n);
+    return map == PassMap::Col && is_smooth(d) ? smooth_line_lpc(d, map) : chain_lines_per_tile(d.n);
 }
 
 cudaError_t launch_chain(const ChainDesc& cd, const void* in, void* out, void* ws, cudaStream_t stream)
@@ -197,16 +189,15 @@ cudaError_t launch_chain(const ChainDesc& cd, const void* in, void* out, void* w
     const ChainFn fn = select(cd.col, cd.row);
     if (fn == nullptr || cd.waves < 1 || cd.col_items < 1 || cd.row_items < 1 || cd.lag < 1 || cd.slots <= cd.lag)
         return cudaErrorInvalidConfiguration;
-    SmoothSides sides{};
-    auto side = [](const PassDesc& d, int lpc, SmoothSched* s, smooth::Tile* t) {
-        if (!is_smooth(d))
-            return lpc * lfft::cta_line_pitch(d.n, lpc) * 8;
-        return smooth_tile(d, lpc, s, t) ? smooth_line_smem(d, lpc) : -1;
-    };
-    const int a = side(cd.col, cd.col_lpc, &sides.col_s, &sides.col_t);
-    const int b = side(cd.row, cd.row_lpc, &sides.row_s, &sides.row_t);
-    if (a < 0 || b < 0)
-        return cudaErrorInvalidConfiguration;
+    SmoothSide side{};
+    int a = cd.col_lpc * lfft::cta_line_pitch(cd.col.n, cd.col_lpc) * 8;
+    if (is_smooth(cd.col))
+    {
+        if (!smooth_tile(cd.col, cd.col_lpc, &side.s, &side.t))
+            return cudaErrorInvalidConfiguration;
+        a = smooth_line_smem(cd.col, cd.col_lpc);
+    }
+    const int b = cd.row_lpc * lfft::cta_line_pitch(cd.row.n, cd.row_lpc) * 8;
     const int smem = a > b ? a : b;
     if (const cudaError_t e = allow_smem(fn, smem); e != cudaSuccess)
         return e;
@@ -214,7 +205,7 @@ cudaError_t launch_chain(const ChainDesc& cd, const void* in, void* out, void* w
     if (total >= 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
     const long long grid = total;
-    fn<<<static_cast<unsigned>(grid), kChainThreads, smem, stream>>>(cd, sides, static_cast<const float2*>(in),
+    fn<<<static_cast<unsigned>(grid), kChainThreads, smem, stream>>>(cd, side, static_cast<const float2*>(in),
                                                                       static_cast<float2*>(out),
                                                                       static_cast<float2*>(ws));
     return cudaGetLastError();

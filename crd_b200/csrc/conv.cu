@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kMaxThreads)
 // The same for a real wavelet: X and K are spectra of real sequences, so w is real and its FFT of n = 2M points is an
 // M-point one (real_pair.cuh): Y = X K at k and M - k, k <= M/2, gives the pairs Q, and conj(FFT(conj Q)) holds
 // w[2m] + i w[2m + 1]. Half the arithmetic and half the shared memory of the complex form, whose 8192-point lines left
-// one 128-register CTA of 256 threads doing one line's stages at a time (64 x 64 lines: 180 -> 98 us a pass); the
+// one 128-register CTA of 256 threads doing one line's stages at a time (64 x 64 lines: 176 -> 92 us a pass); the
 // coefficients' imaginary parts are the exact 0 they stand for.
 template <class S, int P>
 __global__ void __launch_bounds__(256, P == 16 ? 4 : 2)

@@ -100,3 +100,35 @@ def test_chain_wait_runs_out_without_fault(monkeypatch):
     rows = np.array([0, batch - 1])
     want = oracle.fft64(x.cpu().numpy().reshape(batch, n)[rows])
     assert oracle.rel_l2(y.cpu().numpy().reshape(batch, n)[rows], want) <= 1e-6
+
+
+# (n, n1, batch): pairs of schedules that the default splits do not take: 105, 64 and 512 x 1024, 1024 x 512, and
+# run-time-schedule columns (60, 35) over 512-point rows
+FORCED = [(107520, 105, 45), (65536, 64, 80), (1 << 19, 1024, 20), (1 << 19, 512, 20), (30720, 60, 150), (17920, 35, 260)]
+
+
+@pytest.mark.parametrize("n,n1,batch", FORCED)
+@pytest.mark.parametrize("inverse", [False, True])
+def test_chain_of_forced_splits(n, n1, batch, inverse, monkeypatch):
+    from crd_b200._lib import lib
+    from crd_b200.hesap import device_status
+
+    monkeypatch.setenv("CRDFFT_TMA_COL", "0")  # the wave form on the line kernels too
+    assert lib().crdfft_set_decomposition(n, 3, n1) == 0
+    try:
+        ref_plan = _plan(n, batch, False, monkeypatch)
+        plan = _plan(n, batch, True, monkeypatch)
+    finally:
+        lib().crdfft_set_decomposition(n, 0, 0)
+    assert plan.info()["factors"][:2] == [n1, n // n1]
+    x = oracle.lcg_complex64(0xC4A5 ^ n, n * batch).reshape(batch, n)
+    t = torch.from_numpy(x).cuda()
+    ref, out = torch.empty_like(t), torch.empty_like(t)
+    d = cf.INVERSE if inverse else cf.FORWARD
+    ref_plan.execute(t, ref, d)
+    plan.execute(t, out, d)
+    torch.cuda.synchronize()
+    device_status(plan)
+    rows = [0, batch - 1]
+    assert oracle.rel_l2(out.cpu().numpy()[rows], oracle.fft64(x[rows], inverse)) <= 1e-6
+    assert oracle.rel_l2(out.cpu().numpy(), ref.cpu().numpy()) <= 1e-6
