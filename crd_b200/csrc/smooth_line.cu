@@ -234,7 +234,8 @@ int smooth_threads(const SmoothSched& s, int lpc, int smem_bytes, int regs, long
 
 // Lines a CTA: along the lines, tiles of about 2200 points (many CTAs an SM hide each other's phases: 1000-point lines
 // 2 a CTA 68.8 us, 8 74.8); across them, runs of 64 bytes or more as long as a tile fits (2400 points 8 a CTA 110 us, 4
-// 114; 360 points 32 a CTA 66.3, 8 71.5).
+// 114; 360 points 32 a CTA 66.3, 8 71.5). A pass of fewer tiles than SMs takes shorter ones, one an SM: its time is then
+// that of one tile, whose threads do less each (3000 points x 33: 8 a CTA 17.9 us, one 8.3; x 256: 17.0, two 10.2).
 int smooth_line_lpc(const PassDesc& d, PassMap map)
 {
     const bool across = map == PassMap::Col || (d.out.estride != 1 && d.out.ldist == 1 && d.lines_per_group > 1);
@@ -244,6 +245,8 @@ int smooth_line_lpc(const PassDesc& d, PassMap map)
         lpc = d.n <= 400 ? 32 : d.n <= 560 ? 16 : d.n <= 3000 ? 8 : d.n <= 6000 ? 4 : 2;
         while (lpc < 128 && lpc * d.n < 1500)
             lpc *= 2;
+        while (lpc > 1 && d.lines <= 148LL * (lpc / 2))
+            lpc /= 2;
     }
     else
         lpc = std::max(1, 2200 / d.n);

@@ -112,3 +112,15 @@ def test_uneven_items(dev, sizes):
         got = out.cpu().numpy()
         for n, at in list(zip(plan.sizes, plan.offsets))[:8]:
             assert oracle.rel_l2(got[at:at + n], oracle.fft64(x[at:at + n], inverse)) <= 1e-6, n
+
+
+@pytest.mark.parametrize("n,batch", [(6, 149), (60, 148), (100, 149), (360, 297), (1000, 300), (2000, 593), (3125, 75),
+                                     (8000, 33)])
+def test_fewer_tiles_than_sms(dev, n, batch):
+    """Tiles of 1, 2, 4 and 8 lines across a small batch, both sides of the batch that fills the SMs once."""
+    import crd_b200 as cf
+
+    x = oracle.lcg_complex64(n + batch, n * batch).reshape(batch, n)
+    plan = cf.Plan([n], batch=batch, istride=batch, idist=1, ostride=batch, odist=1)
+    got = run(np.ascontiguousarray(x.T), plan, cf.FORWARD).T
+    assert oracle.rel_l2(got, want(x, False)) <= 1e-6
