@@ -737,7 +737,9 @@ bool heuristic_shape(const PassDesc& d, PassMap map, bool dl, bool ds, PassShape
         *out = smooth_shape(d, map, dl, ds);
         return true;
     }
-    const bool want32 = d.n > 8192 || (map == PassMap::Col && d.n >= 1024); // (1024-point columns 0.156 ms, 0.182 at 16)
+    // (1024-point columns: 0.156 ms a 256 MiB batch against 0.182 at 16 points; of one 512-thread tile an SM or less, with
+    // 16 points: 1024 of them 7.1 us against 8.3, 33 7.1 against 8.3; 2048 of them 12.8 against 10.4.)
+    const bool want32 = d.n > 8192 || (map == PassMap::Col && (d.n >= 2048 || (d.n == 1024 && d.lines > 148 * 8)));
     if (want32)
     {
         const PassShape sh = shape_with(d.n, d.nstages, map, dl, ds, 32);
