@@ -981,14 +981,28 @@ bool cluster_ok(const Plan& p, long long n, long long istride, long long idist, 
            p.desc.precision == CRDFFT_PREC_FP32 && cluster_split(n, &a, &b);
 }
 
-Decomp rule_decomp(const Plan& p, long long n, long long istride, long long idist, long long ostride, long long odist)
+// Transforms of up to 2^20 points in all (2^19 of length 2^19), too few tiles to fill the GPU: the split's cost is the
+// latency of the two passes, not their throughput, and 512-point columns before 256 to 1024-point rows have the least
+// (2^18 x 1: 9.4 us as 512 x 512, 11.7 as 256 x 1024; 2^17 x 4: 9.7 as 512 x 256, 10.7 as 128 x 1024; x 8: 13.3 and
+// 12.9, but with a padded distance, which the tensor-copy kernel does not take, 12.5 and 14.2; 2^19 x 1: 9.8 as
+// 512 x 1024, 11.7 as 1024 x 512, x 2: 14.1 and 13.2).
+bool latency_split(long long n, long long batch, long long* n1)
+{
+    if (n * batch > (n < (1LL << 19) ? 1LL << 20 : 1LL << 19) || n % 512 != 0 || n / 512 < 256 || !has_static_schedule(n / 512))
+        return false;
+    *n1 = 512;
+    return true;
+}
+
+Decomp rule_decomp(const Plan& p, long long n, long long batch, long long istride, long long idist, long long ostride,
+                   long long odist)
 {
     if (single_pass_ok(n))
         return Decomp{1, 0};
     if (cluster_ok(p, n, istride, idist, ostride, odist))
         return Decomp{2, 0};
     long long n1 = 0, n2 = 0;
-    if (four_step_split(n, &n1, &n2))
+    if (latency_split(n, batch, &n1) || four_step_split(n, &n1, &n2))
         return Decomp{3, n1};
     return Decomp{0, 0};
 }
@@ -1113,7 +1127,7 @@ Decomp choose_decomp(const Plan& p, long long n, long long batch, long long istr
 {
     if (t_forced != nullptr && t_forced_n == n)
         return *t_forced;
-    Decomp rule = rule_decomp(p, n, istride, idist, ostride, odist);
+    Decomp rule = rule_decomp(p, n, batch, istride, idist, ostride, odist);
     // The half-length transform of an R2C plan: the row pass with the fused recombination (rows of 512 or 1024 points,
     // an even number of them) where the closest-to-square split gives one; it saves a pass over the spectrum.
     long long c1 = 0, c2 = 0;
