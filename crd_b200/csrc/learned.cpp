@@ -34,12 +34,21 @@ Model g_models[2];
 bool g_ready[2] = {false, false};
 const char* const kTags[2] = {"crdfft-mlp", "crdfft-mlp-decomp"};
 
+// Adds one stage's radix to the counts of the factors 16, 8, 4, 2, 3, 5, 7 (24 as 8 and 3, 20 as 4 and 5, 32 as 16 and 2).
+void count_radix(int R, float* f)
+{
+    static const int kFactors[] = {16, 8, 4, 2, 3, 5, 7};
+    for (int i = 0; i < 7; ++i)
+        for (; R % kFactors[i] == 0; R /= kFactors[i])
+            f[i] += 1;
+}
+
 size_t param_count(int d, int h) { return static_cast<size_t>(h) * d + h + static_cast<size_t>(h) * h + h + h + 1; }
 
 } // namespace
 
 // Features of a pass under a launch shape, all O(1) in magnitude:
-//   0 log2 n              1 stages                   2-8 stages of radix 16, 8, 4, 2, 3, 5, 7
+//   0 log2 n              1 stages                   2-8 factors 16, 8, 4, 2, 3, 5, 7 of the stages' radices
 //   9 log2 lines          10 log2 lines a group      11 column map            12 direct load   13 direct store
 //   14 conjugation/scale  15 four-step twiddle       16-17 unit element stride in / out
 //   18-19 log2 element stride in / out               20-21 unit line distance in / out
@@ -54,21 +63,7 @@ void pass_features(const PassDesc& d, const PassShape& sh, float* f)
     f[0] = lg2(d.n);
     f[1] = static_cast<float>(d.nstages);
     for (int s = 0; s < d.nstages; ++s)
-    {
-        switch (d.radix[s])
-        {
-            case 16: f[2] += 1; break;
-            case 8: f[3] += 1; break;
-            case 4: f[4] += 1; break;
-            case 2: f[5] += 1; break;
-            case 3: f[6] += 1; break;
-            case 9: f[6] += 2; break;
-            case 25: f[7] += 2; break;
-            case 5: f[7] += 1; break;
-            case 7: f[8] += 1; break;
-            default: break;
-        }
-    }
+        count_radix(d.radix[s], f + 2);
     f[9] = lg2(static_cast<double>(d.lines));
     f[10] = lg2(static_cast<double>(d.lines_per_group));
     f[11] = sh.map == PassMap::Col ? 1.0f : 0.0f;
@@ -278,7 +273,7 @@ float learned_decomp_predict(const float* feat)
 // Features of a 1-D decomposition choice, all O(1) in magnitude:
 //   0 log2 n              1 log2 batch               2 log2 bytes of input     3-5 single pass / cluster / four-step
 //   6 log2 n1 (columns)   7 log2 n2 (rows)           8 |log2 (n1 / n2)|        9-10 n1, n2 have compile-time schedules
-//   11-17 stages of radix 16, 8, 4, 2, 3, 5, 7 in n1    18-24 the same for n2
+//   11-17 factors 16, 8, 4, 2, 3, 5, 7 of n1's radices  18-24 the same for n2
 //   25 n2 a multiple of 16 (whole column tiles)      26 unit strides and packed  27 padded distances
 //   28 precision (0 FP32, 1 tensor-core form)        29 waves of the four-step at the default wave size (log2)
 //   30 the column pass takes the tensor-copy kernel  31 1 (bias feature, constant)
@@ -299,24 +294,10 @@ void decomp_features(long long n, int kind, long long n1, long long batch, bool 
     f[8] = std::fabs(f[6] - f[7]);
     f[9] = stat1 ? 1.0f : 0.0f;
     f[10] = stat2 ? 1.0f : 0.0f;
-    auto count = [&](const int* r, int s, int at) {
-        for (int i = 0; i < s; ++i)
-            switch (r[i])
-            {
-                case 16: f[at + 0] += 1; break;
-                case 8: f[at + 1] += 1; break;
-                case 4: f[at + 2] += 1; break;
-                case 2: f[at + 3] += 1; break;
-                case 3: f[at + 4] += 1; break;
-                case 9: f[at + 4] += 2; break;
-                case 25: f[at + 5] += 2; break;
-                case 5: f[at + 5] += 1; break;
-                case 7: f[at + 6] += 1; break;
-                default: break;
-            }
-    };
-    count(r1, s1, 11);
-    count(r2, s2, 18);
+    for (int i = 0; i < s1; ++i)
+        count_radix(r1[i], f + 11);
+    for (int i = 0; i < s2; ++i)
+        count_radix(r2[i], f + 18);
     f[25] = (kind == 3 && n2 % 16 == 0) ? 1.0f : 0.0f;
     f[26] = packed_unit ? 1.0f : 0.0f;
     f[27] = padded ? 1.0f : 0.0f;

@@ -1023,8 +1023,8 @@ std::vector<Decomp> decomp_candidates(const Plan& p, long long n, long long istr
         out.push_back(Decomp{1, 0});
     if (cluster_ok(p, n, istride, idist, ostride, odist))
         out.push_back(Decomp{2, 0});
-    // Four-step splits: those whose two line lengths both have compile-time schedules, and the four splits closest
-    // to square among the others (run on the run-time schedule); the rule's own split is always among them.
+    // Four-step splits: those whose two line lengths both have compile-time schedules, and the four cheapest of the
+    // others by the rule's pass costs; the rule's own split is always among them.
     if (n >= 2048 && n < (1LL << 31))
     {
         std::vector<std::pair<double, long long>> other;
@@ -1035,7 +1035,7 @@ std::vector<Decomp> decomp_candidates(const Plan& p, long long n, long long istr
             if (has_static_schedule(a) && has_static_schedule(n / a))
                 out.push_back(Decomp{3, a});
             else
-                other.emplace_back(std::fabs(std::log(static_cast<double>(a) * a / static_cast<double>(n))), a);
+                other.emplace_back(split_pass_cost(a, false, true) + split_pass_cost(n / a, true, true), a);
         }
         std::sort(other.begin(), other.end());
         for (size_t i = 0; i < other.size() && i < 4; ++i)
@@ -1047,10 +1047,14 @@ std::vector<Decomp> decomp_candidates(const Plan& p, long long n, long long istr
     return out;
 }
 
+// The radices the line kernels run for n points.
 void radix_list(long long n, std::vector<int>& r)
 {
     r.clear();
-    radices_for(n, r);
+    if (has_static_schedule(n))
+        radices_for(n, r);
+    else
+        smooth_radices(n, r);
 }
 
 void decomp_feature_vector(const Plan& p, long long n, const Decomp& c, long long batch, bool packed_unit,

@@ -278,3 +278,33 @@ def test_measure_log_carries_features_and_learned_mode_plans_correctly():
         F.set_planner("estimate")
         F.learned_model_forget()
         F.wisdom_forget()
+
+
+@pytest.mark.gpu
+def test_features_name_the_radices_that_run():
+    """The factors that a candidate's features count multiply to its line lengths, composite radices (12, 15, 20 ..)
+    among them: a feature vector of other radices describes kernels that do not run."""
+    import crd_b200 as cf
+    import crd_b200.hesap as F
+    from crd_b200.learned_planner import parse_log
+
+    factors = np.array([16, 8, 4, 2, 3, 5, 7], dtype=float)
+    F.wisdom_forget()
+    F.set_planner("measure")
+    try:
+        cf.Plan([240], batch=300)
+        cf.Plan([3000], batch=30)
+        cf.Plan([100000], batch=4)
+        log = F.planner_log()
+    finally:
+        F.set_planner("estimate")
+        F.wisdom_forget()
+    passes, decomps = parse_log(log), parse_log(log, decomp=True)
+    assert len(passes) >= 4 and len(decomps) >= 1
+    for g in passes:
+        for f in g.feats:
+            assert np.isclose(np.prod(factors ** f[2:9]), 2.0 ** f[0], rtol=1e-4)
+    for g in decomps:
+        for f in g.feats:
+            assert np.isclose(np.prod(factors ** f[11:18]), 2.0 ** f[6], rtol=1e-4)
+            assert np.isclose(np.prod(factors ** f[18:25]), 2.0 ** f[7], rtol=1e-4)
