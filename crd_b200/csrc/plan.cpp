@@ -749,29 +749,24 @@ bool heuristic_shape(const PassDesc& d, PassMap map, bool dl, bool ds, PassShape
             return true;
         }
     }
-    // A compile-time schedule first, at either thread width (the radix-32 schedules exist at 32 points a thread
-    // only: without this order 1024 and 8192 took the run-time kernel at 16 points a thread, 4x slower for 1024),
-    // then the run-time schedule. A four-step row pass the tensor-store kernel takes goes to it (its transposed
-    // store is 40 % of the thread-stored pass's time).
-    for (int pass = 0; pass < 2; ++pass)
-        for (int P : {16, 32})
+    // The compile-time schedule at either thread width (the radix-32 schedules exist at 32 points a thread only). A
+    // four-step row pass the tensor-store kernel takes goes to it (its transposed store is 40 % of the thread-stored
+    // pass's time).
+    for (int P : {16, 32})
+    {
+        PassShape sh = shape_with(d.n, d.nstages, map, dl, ds, P);
+        if (sh.threads_per_line * sh.lines_per_cta > pass_threads_limit(P, d.n) || !pass_has_static(d, P))
+            continue;
+        PassShape t = sh;
+        t.tma_store = true;
+        if (row_tstore_supported(d, t))
         {
-            PassShape sh = shape_with(d.n, d.nstages, map, dl, ds, P);
-            if (sh.threads_per_line * sh.lines_per_cta > pass_threads_limit(P, d.n))
-                continue;
-            if (pass == 0 ? pass_has_static(d, P) : pass_has_kernel(d, sh))
-            {
-                PassShape t = sh;
-                t.tma_store = true;
-                if (pass == 0 && row_tstore_supported(d, t))
-                {
-                    t.smem_bytes = 1024 + t.lines_per_cta * pass_cta_line_pitch(d.n, t.lines_per_cta) * 8;
-                    sh = t;
-                }
-                *out = sh;
-                return true;
-            }
+            t.smem_bytes = 1024 + t.lines_per_cta * pass_cta_line_pitch(d.n, t.lines_per_cta) * 8;
+            sh = t;
         }
+        *out = sh;
+        return true;
+    }
     return false;
 }
 
@@ -1323,8 +1318,6 @@ crdfft_status make_line_step(Plan& p, long long n, long long lines, long long lp
         dl = in.ldist == 1 && lpg > 1;
         ds = out.ldist == 1 && lpg > 1;
     }
-    if (d.nstages == 0) // n == 1: no butterflies; the pass is a copy with the epilogue, staged through smem
-        dl = ds = false;
     // Row lines of 32 points or fewer: one or two threads a line, so a direct load or store would touch a separate
     // 128-byte line per thread; staged through shared memory the CTA's accesses are contiguous.
     if (map == PassMap::Row && n <= 32)
@@ -1630,7 +1623,7 @@ crdfft_status plan_c2c_1d(Plan& p, long long n, long long batch, long long istri
     // L2 waves: a wave small enough that pass 1's output is still in L2 when pass 2 reads it, one workspace slot a
     // lane, consecutive waves round-robin on the plan's internal streams so that one wave's pass 2 overlaps the next
     // one's pass 1 (and fills its tail). Otherwise one large wave at a time on the caller's stream.
-    // (Transforms above 2 MiB are left to large waves: a 24 MiB wave of them is too few tiles to fill the GPU.)
+    // (Transforms above 2 MiB are left to large waves: a 32 MiB wave of them is too few tiles to fill the GPU.)
     const bool l2w = l2_waves() && t_arena == nullptr && n * 8 <= l2_wave_max_transform() &&
                      batch * n * 8 > kL2WavesFrom;
     long long wave = std::max(1LL, (l2w ? l2_wave_bytes() : wave_bytes()) / (n * 8));
