@@ -10,7 +10,8 @@
 //                     The padded sequences stay in L2 (waves of a few tens of MB).
 //
 // Ten and more launches over m = 2^k before (pad, two transforms of two passes and two waves each, product, chirp):
-// 10007 points x 251, m = 32768, 224 us; bound then by the launches' ramps and by L2, now by issued instructions.
+// 10007 points x 251, m = 32768, 226 us; bound then by the launches' ramps and by L2. Now 92 us, bound by latency at 19
+// to 24 warps an SM (39-43 % issue) and by instruction fetch.
 
 #include "kernels.hpp"
 #include "pass_desc.hpp"

@@ -11,19 +11,19 @@
 // Each item is a tile of the run-time-schedule lines (smooth_line.cuh), up to 4096 points: about 35 KB of shared memory
 // and 256 threads at 80 registers, three CTAs an SM, so that one item's loads, stages and stores overlap the others'
 // (20,000 transforms: 1.85 ms; 128 threads and five CTAs 1.96, tiles of 8192 points 1.85 but 60 transforms 25 us
-// instead of 17). CTAs (as
-// many as fit on the GPU at once, G of them) take items in list order, CTA c the items c, c + G, ...; the next item's
-// descriptor, schedule and line offsets come into shared memory while the current one is transformed.
+// instead of 17). CTAs (as many as fit on the GPU at once, G of them) take items in list order, CTA c the items c, c + G,
+// ...; the next item's descriptor, schedule and line offsets come into shared memory while the current one is transformed.
 //
-// A ROW item follows its transform's COL items in the list by more than G items, so they are nearly always done when
-// it starts, and near enough that the intermediate is still in L2 (whose lines the ROW item drops after reading). Its
-// wait on its transform's completion counter always ends: the earliest unfinished item of the list is the next one of
+// While COL items of other transforms remain, a transform's ROW items follow its last COL item by more than G items, so
+// those are nearly always done when it starts, and near enough that the intermediate is still in L2 (whose lines the ROW
+// item drops after reading); the last transforms' ROW items follow the SMALL ones, however few, and may have to wait.
+// A wait on its transform's completion counter always ends: the earliest unfinished item of the list is the next one of
 // its CTA (the CTA's earlier items are earlier in the list), and what it waits for is earlier still. The wait is
 // bounded anyway (spin_limit polls): one that runs out sets the plan's status word and skips the item.
 //
 // Two asynchronously filled 32 KB slots and out-of-place stages before: 215 instructions a point and pass, two CTAs an
-// SM, every intermediate through HBM. Now 95 instructions; bound by latency (42 % issue, the barriers
-// of two or three short stages an item first among the stalls).
+// SM, every intermediate through HBM, 3.63 ms. Now 95 instructions; bound by latency (42 % issue, the barriers of two or
+// three short stages an item first among the stalls).
 
 #include "kernels.hpp"
 #include "smem_limit.hpp"

@@ -7,9 +7,9 @@
 // takes `ppc` consecutive pairs of one signal and writes one row of sums, in a fixed order.
 //
 // The segment-by-segment kernel (spectral.cu) with a half-length real transform issues 104 instructions a complex point,
-// its shared-memory pipe 74 % busy, and leaves a row of sums every few segments for the second launch to add (58 of 606 us
-// for 64 signals x 2^21 samples at 1024). Here 48 instructions a point, 74 %
-// of the issue slots (what bounds it now), and a few dozen rows a signal: 238 us.
+// its shared-memory pipe 74 % busy, and leaves a row of sums every few segments for the second launch to add: 606 us for
+// 64 signals x 2^21 samples at 1024. Here 48 instructions a point, 74 % of the issue slots (what bounds it now), and a
+// few dozen rows a signal: 238 us.
 
 #include "codelets.cuh"
 #include "index.cuh"
