@@ -2709,13 +2709,14 @@ crdfft_status build_uneven(Plan& p, const int64_t* sizes, int64_t count, const i
         st = upload_vec(p, scheds, &u.scheds);
     if (st == CRDFFT_OK)
         st = upload_vec(p, line_off, &u.line_off);
-    std::vector<int> counters(std::max<size_t>(1, large.size()), 0);
+    std::vector<int> counters(1 + large.size(), 0);
     const int* cdev = nullptr;
     if (st == CRDFFT_OK)
         st = upload_vec(p, counters, &cdev);
     if (st != CRDFFT_OK)
         return st;
-    u.done = const_cast<int*>(cdev);
+    u.started = const_cast<int*>(cdev);
+    u.done = u.started + 1;
     u.err = p.err;
     u.nitems = static_cast<int>(items.size());
     u.ntransforms = static_cast<int>(large.size());

@@ -42,7 +42,8 @@ struct UnevenDesc
     const UnevenItem* items;
     const SmoothSched* scheds; // one per line length
     const long long* line_off;
-    int* done;      // COL items finished, per long transform (zeroed before each launch)
+    int* started;   // CTAs started, and behind it done (both zeroed before a launch with long transforms)
+    int* done;      // COL items finished, per long transform
     int* err;
     int nitems;
     int ntransforms;

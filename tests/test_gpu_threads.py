@@ -61,3 +61,30 @@ def test_two_threads(make):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_uneven_beside_other_kernels():
+    """Uneven batches with long transforms (row tiles wait for column tiles) on three streams of different priority at
+    once, among launches that come and go: whatever part of each grid is resident, every wait ends and the results are
+    those of a batch alone."""
+    from crd_b200.hesap import device_status
+
+    jobs = []
+    for i, sizes in enumerate(([65536] * 40 + [3000] * 30, [4200] * 200 + [16] * 500, [20000] * 90)):
+        plan = cf.UnevenPlan(sizes)
+        x = torch.from_numpy(oracle.lcg_complex64(31 + i, plan.total)).cuda()
+        want = torch.zeros_like(x)
+        plan.execute(x, want)
+        jobs.append((plan, x, want, torch.zeros_like(x), torch.cuda.Stream(priority=-i)))
+    other = torch.rand(1 << 24, device="cuda")
+    side = torch.cuda.Stream(priority=-1)
+    torch.cuda.synchronize()
+    for _ in range(60):
+        with torch.cuda.stream(side):
+            other.mul_(1.0)
+        for plan, x, _, out, stream in jobs:
+            plan.execute(x, out, cf.FORWARD, stream)
+    torch.cuda.synchronize()
+    for plan, _, want, out, _ in jobs:
+        device_status(plan)
+        assert torch.equal(out, want)
