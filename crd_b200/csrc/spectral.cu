@@ -231,46 +231,65 @@ __global__ void __launch_bounds__(DYN ? kMaxThreads : kStaticThreads, DYN ? 1 : 
     }
 }
 
-// The per-CTA sums of each signal added in a fixed order, divided by the segment count (spectral.hpp:158-171): `slices`
-// of consecutive rows, each in row order, then the slices in order (finish_slices).
+// The per-CTA sums of each signal added in a fixed order, divided by the segment count (spectral.hpp:158-171): eight
+// slices of consecutive rows, each in row order, then the slices in order. `lanes` threads share a frequency's slices.
 constexpr int kFinishThreads = 256;
+constexpr int kFinishSlices = 8;
 __global__ void __launch_bounds__(kFinishThreads)
     welch_finish_kernel(const float* __restrict__ part, float* __restrict__ psd, long long count, int ntiles, int nfreq,
-                        float nseg, int slices)
+                        float nseg, int lanes)
 {
-    __shared__ float sums[kFinishThreads];
-    const int freqs = kFinishThreads / slices; // a CTA's frequencies
-    const int slice = threadIdx.x / freqs;
-    const int k0 = threadIdx.x - slice * freqs;
+    __shared__ float sums[kFinishSlices * kFinishThreads];
+    const int freqs = kFinishThreads / lanes; // a CTA's frequencies
+    const int lane = threadIdx.x / freqs;
+    const int k0 = threadIdx.x - lane * freqs;
     const long long idx = static_cast<long long>(blockIdx.x) * freqs + k0;
     const bool ok = idx < count * nfreq;
-    float acc = 0.0f;
     if (ok)
     {
         const long long g = idiv(idx, nfreq);
         const int k = static_cast<int>(idx - g * nfreq);
         const float* p = part + g * ntiles * static_cast<long long>(nfreq) + k;
-        const int each = (ntiles + slices - 1) / slices;
-        const int end = min(ntiles, (slice + 1) * each);
-        for (int t = slice * each; t < end; ++t)
-            acc += p[static_cast<long long>(t) * nfreq];
+        const int each = (ntiles + kFinishSlices - 1) / kFinishSlices;
+        auto slice = [&](int s) {
+            const int end = min(ntiles, (s + 1) * each);
+            float acc = 0.0f;
+            for (int t = s * each; t < end; ++t)
+                acc += p[static_cast<long long>(t) * nfreq];
+            return acc;
+        };
+        if (lanes == 1)
+        {
+            float acc = slice(0);
+            for (int s = 1; s * each < ntiles; ++s)
+                acc += slice(s);
+            psd[idx] = acc / nseg;
+        }
+        else
+        {
+            const int mine = kFinishSlices / lanes;
+            for (int s = lane * mine; s < (lane + 1) * mine; ++s)
+                sums[s * freqs + k0] = slice(s);
+        }
     }
-    sums[threadIdx.x] = acc;
-    __syncthreads();
-    if (slice != 0 || !ok)
+    if (lanes == 1)
         return;
-    for (int s = 1; s < slices; ++s)
+    __syncthreads();
+    if (lane != 0 || !ok)
+        return;
+    float acc = sums[k0];
+    for (int s = 1; s < kFinishSlices; ++s)
         acc += sums[s * freqs + k0];
     psd[idx] = acc / nseg;
 }
 
-// Slices of a signal's rows: as many, up to eight of four rows or more, as fill the device (148 x 2048 threads) when the
-// frequencies alone do not: 16 signals x 1024 rows of 513 took 58 us as one slice, most of the device idle; 2000 signals
-// x 1 row of 2049 took 248 us with the transforms when every row had eight slices, seven of them empty, and take 86.
-int finish_slices(long long freqs, int ntiles)
+// Threads a frequency: as many, up to a slice each, as have rows and fill the device (148 x 2048 threads) when the
+// frequencies alone do not: 16 signals x 1024 rows of 513 took 58 us with one, most of the device idle; 2000 signals
+// x 1 row of 2049 took 248 us with the transforms when every frequency had eight, seven of them idle, and take 86.
+int finish_lanes(long long freqs, int ntiles)
 {
     int s = 1;
-    while (s < 8 && ntiles >= 8 * s && freqs * s < 148LL * 2048)
+    while (s < kFinishSlices && ntiles > s && freqs * s < 148LL * 2048)
         s *= 2;
     return s;
 }
@@ -361,14 +380,14 @@ cudaError_t launch_welch_finish(const SpectralDesc& sd, const void* part, void* 
     const long long total = sd.count * nfreq;
     if (total <= 0)
         return cudaSuccess;
-    const int slices = lfft::finish_slices(total, sd.ntiles);
-    const long long freqs = lfft::kFinishThreads / slices;
+    const int lanes = lfft::finish_lanes(total, sd.ntiles);
+    const long long freqs = lfft::kFinishThreads / lanes;
     const long long blocks = (total + freqs - 1) / freqs;
     if (blocks > 0x7fffffffLL)
         return cudaErrorInvalidConfiguration;
     lfft::welch_finish_kernel<<<static_cast<unsigned>(blocks), lfft::kFinishThreads, 0, stream>>>(
         static_cast<const float*>(part), static_cast<float*>(psd), sd.count, sd.ntiles, nfreq,
-        static_cast<float>(sd.nseg), slices);
+        static_cast<float>(sd.nseg), lanes);
     return cudaGetLastError();
 }
 
