@@ -251,26 +251,50 @@ __global__ void __launch_bounds__(kFinishThreads)
         const int k = static_cast<int>(idx - g * nfreq);
         const float* p = part + g * ntiles * static_cast<long long>(nfreq) + k;
         const int each = (ntiles + kFinishSlices - 1) / kFinishSlices;
-        auto slice = [&](int s) {
-            const int end = min(ntiles, (s + 1) * each);
-            float acc = 0.0f;
-            for (int t = s * each; t < end; ++t)
-                acc += p[static_cast<long long>(t) * nfreq];
-            return acc;
+        if (each == 1) // a row a slice (and one thread: finish_lanes): the rows in order
+        {
+            float sum = 0.0f;
+            for (int t = 0; t < ntiles; ++t)
+                sum += p[static_cast<long long>(t) * nfreq];
+            psd[idx] = sum / nseg;
+            return;
+        }
+        const int mine = kFinishSlices / lanes;
+        // This thread's slices: their rows are one run, eight of them loaded ahead of the sums.
+        int s = lane * mine, left = each;
+        const int end = min(ntiles, (s + mine) * each);
+        float acc = 0.0f, whole = 0.0f;
+        auto close = [&]() {
+            if (lanes == 1)
+                whole += acc;
+            else
+                sums[s * freqs + k0] = acc;
+            ++s;
+            acc = 0.0f;
+            left = each;
         };
+        for (int t = s * each; t < end; t += 8)
+        {
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                v[j] = t + j < end ? __ldg(p + static_cast<long long>(t + j) * nfreq) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (t + j < end)
+                {
+                    acc += v[j];
+                    if (--left == 0)
+                        close();
+                }
+        }
+        if (left != each)
+            close();
         if (lanes == 1)
-        {
-            float acc = slice(0);
-            for (int s = 1; s * each < ntiles; ++s)
-                acc += slice(s);
-            psd[idx] = acc / nseg;
-        }
+            psd[idx] = whole / nseg;
         else
-        {
-            const int mine = kFinishSlices / lanes;
-            for (int s = lane * mine; s < (lane + 1) * mine; ++s)
-                sums[s * freqs + k0] = slice(s);
-        }
+            while (s < (lane + 1) * mine)
+                close();
     }
     if (lanes == 1)
         return;
@@ -283,13 +307,14 @@ __global__ void __launch_bounds__(kFinishThreads)
     psd[idx] = acc / nseg;
 }
 
-// Threads a frequency: as many, up to a slice each, as have rows and fill the device (148 x 2048 threads) when the
-// frequencies alone do not: 16 signals x 1024 rows of 513 took 58 us with one, most of the device idle; 2000 signals
-// x 1 row of 2049 took 248 us with the transforms when every frequency had eight, seven of them idle, and take 86.
+// Threads a frequency: up to a slice each, of 32 rows or more while the frequencies alone leave half the device idle
+// (148 x 1024 threads), of eight while they leave most of it. 16 signals x 1024 rows of 513 took 58 us with one thread a
+// frequency; 2000 signals x 1 row of 2049 248 us with the transforms when every frequency had eight, seven of them idle,
+// now 86; 64 signals x 14 rows of 1025 alone 9.7 us with eight, 7.8 with two, 5.3 with one.
 int finish_lanes(long long freqs, int ntiles)
 {
     int s = 1;
-    while (s < kFinishSlices && ntiles > s && freqs * s < 148LL * 2048)
+    while (s < kFinishSlices && ((ntiles >= 64 * s && freqs * s < 148LL * 1024) || (ntiles >= 16 * s && freqs * s < 148LL * 128)))
         s *= 2;
     return s;
 }
