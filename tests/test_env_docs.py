@@ -1,4 +1,4 @@
-"""Every environment variable of the table in INTEGRATION.md is read by the library, and every one the library reads is
+"""Every environment variable in the integration guide's table is read by the library, and every one the library reads is
 in the table."""
 
 import glob
