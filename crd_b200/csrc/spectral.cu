@@ -308,13 +308,14 @@ __global__ void __launch_bounds__(kFinishThreads)
 }
 
 // Threads a frequency: up to a slice each, of 32 rows or more while the frequencies alone leave half the device idle
-// (148 x 1024 threads), of eight while they leave most of it. 16 signals x 1024 rows of 513 took 58 us with one thread a
-// frequency; 2000 signals x 1 row of 2049 248 us with the transforms when every frequency had eight, seven of them idle,
-// now 86; 64 signals x 14 rows of 1025 alone 9.7 us with eight, 7.8 with two, 5.3 with one.
+// (148 x 1024 threads), of eight while they leave seven eighths idle. 16 signals x 1024 rows of 513 took 58 us with one
+// thread a frequency; 2000 signals x 1 row of 2049 248 us with the transforms when every frequency had eight, seven of
+// them idle, now 86; 64 signals x 14 rows of 1025 alone 9.7 us with eight, 7.8 with two, 5.3 with one.
 int finish_lanes(long long freqs, int ntiles)
 {
     int s = 1;
-    while (s < kFinishSlices && ((ntiles >= 64 * s && freqs * s < 148LL * 1024) || (ntiles >= 16 * s && freqs * s < 148LL * 128)))
+    while (s < kFinishSlices &&
+           ((ntiles >= 64 * s && freqs * s < 148LL * 1024) || (ntiles >= 16 * s && freqs * s < 148LL * 256)))
         s *= 2;
     return s;
 }
